@@ -39,6 +39,7 @@ struct Member {
 struct Bucket {
     RowTile tile{};
     int grid = 0;
+    int groups = 1;          // row groups per CTA
     bool stage = false;
     int max_n = 0, max_pts = 0, kind = 0;
     Task* d_gen = nullptr;   // generation / NSGA offspring tasks
@@ -113,14 +114,11 @@ static int32_t upload_tasks(Group& g, const std::vector<Task>& t, Task** out) {
 
 // build buckets for descriptors [d0, d1) (all of one kind)
 static int32_t build_buckets(Group& g, int d0, int d1, bool nsga, std::vector<Bucket>* out) {
-    std::map<std::pair<int, int>, std::vector<int>> by_tile;
-    for (int i = d0; i < d1; ++i) {
-        const RowTile t = pick_tile(g.hd[i].n);
-        by_tile[{t.block, t.groups}].push_back(i);
-    }
+    std::map<std::pair<int, int>, std::vector<int>> by_tile;  // (threads per row, class of kinds)
+    for (int i = d0; i < d1; ++i) by_tile[{pick_tile(g.hd[i].n).block, row_class(g.hd[i].kind)}].push_back(i);
     for (auto& kv : by_tile) {
         Bucket b;
-        b.tile = RowTile{kv.first.first, kv.first.second};
+        b.tile = RowTile{kv.first.first, 1};
         int kind = 0;
         for (int i : kv.second) {
             const PopDesc& d = g.hd[i];
@@ -133,9 +131,10 @@ static int32_t build_buckets(Group& g, int d0, int d1, bool nsga, std::vector<Bu
         }
         b.kind = kind;
         b.stage = stage_fits(b.tile, b.max_n, b.max_pts, kind);
-        const size_t smem = row_smem_bytes(b.tile, b.max_n, b.max_pts, kind, b.stage);
+        b.groups = row_groups_shared(b.tile, b.max_n, b.max_pts, kind, b.stage);
+        const size_t smem = row_smem_bytes(b.tile, b.max_n, b.max_pts, kind, b.stage, b.groups);
         int per_sm = 0;
-        cudaError_t e = prepare_rows(b.tile, smem, &per_sm);
+        cudaError_t e = prepare_rows(b.tile, kind, b.groups, smem, &per_sm);
         if (e != cudaSuccess || per_sm <= 0) return fail(BRKGA_ERR_UNSUPPORTED, "row kernel does not fit");
         b.grid = per_sm * device_sm_count();
         // each population's rows stay together: its children, then its elite copies
@@ -164,15 +163,16 @@ static RowLaunch bucket_launch(const Group& g, const Bucket& b, int mode, bool a
     L.mode = mode;
     L.tasks = all ? b.d_all : b.d_gen;
     L.ntasks = all ? b.nt_all : b.nt_gen;
-    // groups of consecutive rows per CTA visit, while every CTA keeps work
-    L.task_group = std::max(1, std::min(g.task_group, L.ntasks / std::max(1, b.grid)));
+    // units of consecutive rows per CTA visit: a row for every group of the CTA, several while
+    // every CTA keeps work; batches deal them from the work counter (L.work), the server's
+    // mix statically
+    const int rounds = std::max(1, std::min(g.task_group / b.groups, L.ntasks / std::max(1, b.grid * b.groups)));
+    L.groups_per_cta = b.groups;
+    L.task_group = b.groups * rounds;
     L.max_n = b.max_n;
     L.max_points = b.max_pts;
     L.stage_xy = b.stage ? 1 : 0;
-    // rows dealt from the work counter when a CTA takes several at a time (a batch: +8 %
-    // on 256 island instances); one row per grab (the server's mix) costs more than it
-    // balances (-4 %), so those launches deal statically
-    L.work = (L.task_group > 1) ? g.work : nullptr;
+    L.work = (g.task_group > 1) ? g.work : nullptr;
     return L;
 }
 
@@ -420,8 +420,10 @@ static cudaError_t init_members(Group& g, const std::vector<Member*>& ms) {
         const RowTile t = pick_tile(m->sh.n);
         const int pts = points_of(*m->pd);
         const bool stage = stage_fits(t, m->sh.n, pts, m->pd->kind);
+        const int groups = row_groups_per_cta(t, m->sh.n, pts, m->pd->kind, stage, m->sh.Pi);
         int per_sm = 0;
-        if ((e = prepare_rows(t, row_smem_bytes(t, m->sh.n, pts, m->pd->kind, stage), &per_sm)) != cudaSuccess)
+        if ((e = prepare_rows(t, m->pd->kind, groups, row_smem_bytes(t, m->sh.n, pts, m->pd->kind, stage, groups),
+                              &per_sm)) != cudaSuccess)
             return e;
         for (int i = 0; i < m->ndesc; ++i) {
             RowLaunch L;
@@ -432,6 +434,7 @@ static cudaError_t init_members(Group& g, const std::vector<Member*>& ms) {
             L.max_n = m->sh.n;
             L.max_points = pts;
             L.stage_xy = stage ? 1 : 0;
+            L.groups_per_cta = groups;
             if ((e = launch_rows(L, m->pd->kind, t, per_sm * device_sm_count(), g.stream)) != cudaSuccess) return e;
         }
         if (m->sh.mo) {

@@ -219,7 +219,7 @@ int points_of(const ProblemData& pd) {
 }
 
 bool stage_fits(const RowTile& t, int n, int pts, int kind) {
-    return row_smem_bytes(t, n, pts, kind, true) <= kMaxSmem;
+    return row_smem_bytes(t, n, pts, kind, true, 1) <= kMaxSmem;
 }
 
 // ---------------------------------------------------------------------------------------
@@ -275,14 +275,15 @@ void tune_store(int kind, int n, int rows, const RowTile& t) {
     }
 }
 
-int32_t tile_setup(const RowTile& t, int kind, int n, int pts, TunedTile* out) {
+int32_t tile_setup(const RowTile& t, int kind, int n, int pts, int rows, TunedTile* out) {
     TunedTile tt;
     tt.tile = t;
     tt.stage = stage_fits(t, n, pts, kind);
-    const size_t smem = row_smem_bytes(t, n, pts, kind, tt.stage);
+    tt.groups_per_cta = row_groups_per_cta(t, n, pts, kind, tt.stage, rows);
+    const size_t smem = row_smem_bytes(t, n, pts, kind, tt.stage, tt.groups_per_cta);
     if (smem > kMaxSmem) return fail(BRKGA_ERR_UNSUPPORTED, "tile needs too much shared memory");
     int per_sm = 0;
-    cudaError_t e = prepare_rows(t, smem, &per_sm);
+    cudaError_t e = prepare_rows(t, kind, tt.groups_per_cta, smem, &per_sm);
     if (e != cudaSuccess) {
         cudaGetLastError();
         return cuda_fail(e, "tile set-up");

@@ -110,6 +110,7 @@ struct brkga_engine {
     int nt_gen = 0, nt_all = 0;
     RowTile tile{};
     int grid = 0;
+    int groups_per_cta = 1;
     bool stage = false;
     uint32_t gen = 0;
     bool initialized = false;
@@ -145,6 +146,8 @@ static RowLaunch base_launch(brkga_engine* e, int mode) {
     L.max_n = e->pop.sh.n;
     L.max_points = points_of(*e->pop.pd);
     L.stage_xy = e->stage ? 1 : 0;
+    L.groups_per_cta = e->groups_per_cta;
+    L.task_group = e->groups_per_cta;  // islands: units of a row for every group
     L.gscratch = e->gscratch;
     L.gstride = e->gstride;
     return L;
@@ -402,6 +405,8 @@ int32_t brkga_create(brkga_problem* pbh, const brkga_params* params, brkga_engin
             L.max_n = sh.n;
             L.max_points = pts;
             L.stage_xy = tt.stage ? 1 : 0;
+            L.groups_per_cta = tt.groups_per_cta;
+            L.task_group = tt.groups_per_cta;
             return launch_rows(L, pd->kind, tt.tile, tt.grid, e->stream);
         };
         const int rows = sh.mo ? sh.Pi : e->nt_all;
@@ -424,6 +429,7 @@ int32_t brkga_create(brkga_problem* pbh, const brkga_params* params, brkga_engin
             }
             e->tile = tt.tile;
             e->grid = tt.grid;
+            e->groups_per_cta = tt.groups_per_cta;
             e->stage = tt.stage;
         }
     }
@@ -433,7 +439,7 @@ int32_t brkga_create(brkga_problem* pbh, const brkga_params* params, brkga_engin
         return cuda_fail(err, "sort set-up");
     }
     if (sh.mo) {
-        st = nsga_setup(e->nsga, e->pop, e->dd, e->hd[0], e->tile, e->grid, e->stage);
+        st = nsga_setup(e->nsga, e->pop, e->dd, e->hd[0], e->tile, e->grid, e->groups_per_cta, e->stage);
         if (st != BRKGA_OK) {
             destroy_engine(e);
             return st;

@@ -92,13 +92,14 @@ uint32_t prob_threshold(double p);
 struct TunedTile {
     RowTile tile{};
     int grid = 0;
+    int groups_per_cta = 1;
     bool stage = false;
 };
 template <typename F>
 int32_t autotune_tile(int kind, int n, int pts, int rows, cudaStream_t stream, F&& launch, TunedTile* out);
 int32_t tune_lookup(int kind, int n, int rows, RowTile* t);
 void tune_store(int kind, int n, int rows, const RowTile& t);
-int32_t tile_setup(const RowTile& t, int kind, int n, int pts, TunedTile* out);
+int32_t tile_setup(const RowTile& t, int kind, int n, int pts, int rows, TunedTile* out);
 
 // validated, per-island GA shape
 struct Shape {
@@ -140,9 +141,9 @@ struct Population {
 template <typename F>
 int32_t autotune_tile(int kind, int n, int pts, int rows, cudaStream_t stream, F&& launch, TunedTile* out) {
     RowTile forced{};
-    if (tune_lookup(kind, n, rows, &forced) == BRKGA_OK) return tile_setup(forced, kind, n, pts, out);
-    RowTile cand[16];
-    const int nc = tile_candidates(n, cand, 16);
+    if (tune_lookup(kind, n, rows, &forced) == BRKGA_OK) return tile_setup(forced, kind, n, pts, rows, out);
+    RowTile cand[24];
+    const int nc = tile_candidates(n, cand, 24);
     cudaEvent_t a, b;
     cudaEventCreate(&a);
     cudaEventCreate(&b);
@@ -153,7 +154,7 @@ int32_t autotune_tile(int kind, int n, int pts, int rows, cudaStream_t stream, F
     TunedTile best, deft;
     for (int c = 0; c < nc; ++c) {
         TunedTile tt;
-        if (tile_setup(cand[c], kind, n, pts, &tt) != BRKGA_OK) continue;
+        if (tile_setup(cand[c], kind, n, pts, rows, &tt) != BRKGA_OK) continue;
         if (launch(tt) != cudaSuccess) continue;  // warm-up
         float ms = 1e30f;
         for (int r = 0; r < 3; ++r) {

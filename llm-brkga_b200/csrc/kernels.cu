@@ -24,50 +24,8 @@
 
 namespace bk {
 
-// ---------------------------------------------------------------------------------------
-// shared-memory carve-up for the row kernel
-// ---------------------------------------------------------------------------------------
-struct RowSmem {
-    uint32_t* cnt;            // bucket counters / offsets, NB + 1
-    unsigned long long* sc;   // scattered (okey << 32 | index) composites, n
-    int32_t* perm;            // decoded permutation, n
-    float* xy;                // staged coordinates (1 or 2 sets)
-};
-
 __host__ __device__ inline size_t align_up(size_t x, size_t a) { return (x + a - 1) / a * a; }
 
-// bucket counters: 4 * groups * block buckets (>= n) plus a sentinel, padded to 16 bytes
-__host__ __device__ inline size_t cnt_words(int block, int groups) { return (size_t)4 * groups * block + 4; }
-
-constexpr size_t kRowSmemCap = 227 * 1024;  // opt-in dynamic shared memory per CTA
-
-size_t row_smem_bytes(const RowTile& t, int max_n, int max_points, int kind, bool stage_xy) {
-    size_t b = align_up(cnt_words(t.block, t.groups) * 4, 16);
-    b += align_up((size_t)max_n * 8, 16);
-    b += align_up((size_t)max_n * 4, 16);
-    if (stage_xy && (kind == TSP_COORDS || kind == BITSP_COORDS))
-        b += (size_t)max_points * 8 * (kind == BITSP_COORDS ? 2 : 1);
-    return b;
-}
-
-__device__ __forceinline__ RowSmem carve(unsigned char* base, int block, int groups, int max_n, int max_points) {
-    RowSmem s;
-    size_t off = 0;
-    s.cnt = reinterpret_cast<uint32_t*>(base + off);
-    off += align_up(cnt_words(block, groups) * 4, 16);
-    s.sc = reinterpret_cast<unsigned long long*>(base + off);
-    off += align_up((size_t)max_n * 8, 16);
-    s.perm = reinterpret_cast<int32_t*>(base + off);
-    off += align_up((size_t)max_n * 4, 16);
-    s.xy = reinterpret_cast<float*>(base + off);
-    (void)max_points;
-    return s;
-}
-
-// ---------------------------------------------------------------------------------------
-// decode: stable argsort of one row held in registers (k[g][l] is key index
-// 4 * (threadIdx.x + g * BLOCK) + l)
-// ---------------------------------------------------------------------------------------
 __device__ __forceinline__ int bucket_of(float key, float nbf, int nb) {
     // monotone in okey order: negatives -> 0; [0,1) -> floor(key * nb); >= 1, +inf, NaN -> nb-1
     if (!(key >= 0.0f)) return (key != key) ? nb - 1 : 0;
@@ -126,113 +84,13 @@ __device__ void block_sort_u64(unsigned long long* a, int n) {
 }
 
 // the permutation of a heavy row: each segment's composites sorted, then their indices;
-// called rather than inlined, so the row kernels keep their registers for the common path
+// called rather than inlined, so the kernel keeps its registers for the common path
 template <int BLOCK>
 __device__ __noinline__ void heavy_row_perm(unsigned long long* sc, int32_t* perm, int n, int split) {
     block_sort_u64<BLOCK>(sc, split);
     if (split < n) block_sort_u64<BLOCK>(sc + split, n - split);
     for (int p = threadIdx.x; p < n; p += BLOCK) perm[p] = (int32_t)(uint32_t)sc[p];
     __syncthreads();
-}
-
-// Counters must be zero on entry; they are left holding bucket offsets (the caller
-// re-zeroes them while it no longer needs them).  Bucket count NB = 4 * G * BLOCK >= n,
-// thread t owns the contiguous buckets [4Gt, 4Gt + 4G) for the scan.
-// Keys [split, n) form a second segment sorted on its own (TSPJ's job keys after its city
-// keys): it takes the upper half of the buckets, so no bucket mixes the segments and
-// positions [split, n) of the permutation hold the second segment's order.  A heavy row
-// sorts each segment's composites on its own: the scatter has put the first segment's in
-// [0, split).
-template <int BLOCK, int G>
-__device__ void row_argsort(const float (&k)[G][4], int n, int split, const RowSmem& s, uint32_t* warp_tot) {
-    constexpr int KB = 4 * G, NB = KB * BLOCK;
-    const int t = threadIdx.x;
-    const int nbs = (split < n) ? NB / 2 : NB;
-    const float nbf = (float)nbs;
-    uint32_t bs[G][4];  // (bucket << 16) | slot
-#pragma unroll
-    for (int g = 0; g < G; ++g)
-#pragma unroll
-        for (int l = 0; l < 4; ++l) {
-            const int i = 4 * (t + g * BLOCK) + l;
-            if (i < n) {
-                const int b = bucket_of(k[g][l], nbf, nbs) + ((i >= split) ? nbs : 0);
-                const uint32_t slot = atomicAdd(&s.cnt[b], 1u);
-                bs[g][l] = ((uint32_t)b << 16) | slot;
-            }
-        }
-    __syncthreads();
-    uint4 c[G];
-    uint32_t sum = 0, big = 0;
-#pragma unroll
-    for (int g = 0; g < G; ++g) {
-        c[g] = reinterpret_cast<const uint4*>(s.cnt)[t * G + g];
-        sum += c[g].x + c[g].y + c[g].z + c[g].w;
-        big = max(big, max(max(c[g].x, c[g].y), max(c[g].z, c[g].w)));
-    }
-    uint32_t run = block_exclusive_scan<BLOCK>(sum, warp_tot, nullptr);
-#pragma unroll
-    for (int g = 0; g < G; ++g) {
-        uint4 o;
-        o.x = run;
-        o.y = o.x + c[g].x;
-        o.z = o.y + c[g].y;
-        o.w = o.z + c[g].z;
-        run = o.w + c[g].w;
-        reinterpret_cast<uint4*>(s.cnt)[t * G + g] = o;
-    }
-    if (t == 0) s.cnt[NB] = (uint32_t)n;
-    const bool heavy = __syncthreads_or(big > kHeavyBucket) != 0;
-    // scatter composites
-#pragma unroll
-    for (int g = 0; g < G; ++g)
-#pragma unroll
-        for (int l = 0; l < 4; ++l) {
-            const int i = 4 * (t + g * BLOCK) + l;
-            if (i < n) {
-                const uint32_t b = bs[g][l] >> 16, slot = bs[g][l] & 0xFFFFu;
-                s.sc[s.cnt[b] + slot] = ((unsigned long long)okey(k[g][l]) << 32) | (uint32_t)i;
-            }
-        }
-    __syncthreads();
-    if (heavy) {
-        heavy_row_perm<BLOCK>(s.sc, s.perm, n, split);
-        return;
-    }
-    // exact rank inside the bucket
-#pragma unroll
-    for (int g = 0; g < G; ++g)
-#pragma unroll
-        for (int l = 0; l < 4; ++l) {
-            const int i = 4 * (t + g * BLOCK) + l;
-            if (i < n) {
-                const uint32_t b = bs[g][l] >> 16;
-                const uint32_t b0 = s.cnt[b], b1 = s.cnt[b + 1];
-                const unsigned long long me = ((unsigned long long)okey(k[g][l]) << 32) | (uint32_t)i;
-                uint32_t r = b0;
-                if constexpr (G > 1) {
-                    // long rows: buckets of up to four keys (nearly all of them for keys in
-                    // [0,1)) take predicated steps without a loop, larger ones continue in
-                    // the loop (TSP n = 5000 and knapsack n = 10 000 rows 3 % faster; the
-                    // one-group tiles measured 1 % slower with it and keep the plain loop)
-#pragma unroll
-                    for (uint32_t u = 0; u < 4; ++u)
-                        if (b0 + u < b1) r += (s.sc[b0 + u] < me) ? 1u : 0u;
-                    for (uint32_t q = b0 + 4; q < b1; ++q) r += (s.sc[q] < me) ? 1u : 0u;
-                } else {
-                    for (uint32_t q = b0; q < b1; ++q) r += (s.sc[q] < me) ? 1u : 0u;
-                }
-                s.perm[r] = i;
-            }
-        }
-    __syncthreads();
-}
-
-// zero the bucket counters (4 * G * BLOCK + 1 words) with 128-bit stores
-template <int BLOCK, int G>
-__device__ __forceinline__ void zero_counters(const RowSmem& s) {
-    uint4* c = reinterpret_cast<uint4*>(s.cnt);
-    for (int i = threadIdx.x; i < G * BLOCK + 1; i += BLOCK) c[i] = make_uint4(0u, 0u, 0u, 0u);
 }
 
 // ---------------------------------------------------------------------------------------
@@ -416,14 +274,6 @@ __device__ float knap_greedy(const int32_t* perm, int n, const int2* __restrict_
     return (float)(v0 + vt);
 }
 
-// the same, called rather than inlined: in the one-group row kernels (48 registers) an
-// inlined copy spills registers on every kind's path
-template <int BLOCK>
-__device__ __noinline__ float knap_greedy_call(const int32_t* perm, int n, const int2* __restrict__ items,
-                                               long long C, long long* red, long long* shared_misc, int2* wv) {
-    return knap_greedy<BLOCK>(perm, n, items, C, red, shared_misc, wv);
-}
-
 // TSPJ makespan (configs/tspj_config.hpp:555-585): the city tour from the depot (node 0)
 // and back; at each position the arrival time plus the duration of the job type assigned
 // to that position; the larger of the tour length and the latest job completion.  perm[0,
@@ -451,50 +301,6 @@ __device__ float tspj_makespan(const int32_t* perm, int nc, const float* __restr
             for (int q = 0; q < cnt; ++q) {
                 run = __fadd_rn(run, __shfl_sync(0xffffffffu, e, q));
                 const float jc = __fadd_rn(run, __shfl_sync(0xffffffffu, jd, q));
-                mjc = (mjc < jc) ? jc : mjc;
-            }
-        }
-        const float tt = __fadd_rn(run, __ldg(travel + (size_t)(perm[nc - 1] + 1) * D));
-        if (lane == 0) red[0] = (tt < mjc) ? mjc : tt;
-    }
-    __syncthreads();
-    const float v = red[0];
-    __syncthreads();
-    return v;
-}
-
-// The same for tours of up to 128 cities, called rather than inlined (one-group row
-// kernels): every lane issues the loads of all its positions before the first sequential
-// step, so the walk waits for one round of loads instead of one per 32 cities.
-template <int BLOCK>
-__device__ __noinline__ float tspj_makespan_call(const int32_t* perm, int nc, const float* __restrict__ travel,
-                                                 const float* __restrict__ jobs, float* red) {
-    constexpr int kChunks = 4;
-    if (nc > 32 * kChunks) return tspj_makespan<BLOCK>(perm, nc, travel, jobs, red);
-    const int lane = threadIdx.x & 31;
-    if (threadIdx.x < 32) {
-        const size_t D = (size_t)nc + 1;
-        float e[kChunks], jd[kChunks];
-#pragma unroll
-        for (int c = 0; c < kChunks; ++c) {
-            const int i = 32 * c + lane;
-            e[c] = 0.0f;
-            jd[c] = 0.0f;
-            if (i < nc) {
-                const int city = perm[i] + 1;
-                const int prev = (i == 0) ? 0 : perm[i - 1] + 1;
-                const int job = perm[nc + i] - nc + 1;
-                e[c] = __ldg(travel + (size_t)prev * D + city);
-                jd[c] = __ldg(jobs + (size_t)city * D + job);
-            }
-        }
-        float run = 0.0f, mjc = 0.0f;
-#pragma unroll
-        for (int c = 0; c < kChunks; ++c) {
-            const int cnt = min(32, nc - 32 * c);
-            for (int q = 0; q < cnt; ++q) {
-                run = __fadd_rn(run, __shfl_sync(0xffffffffu, e[c], q));
-                const float jc = __fadd_rn(run, __shfl_sync(0xffffffffu, jd[c], q));
                 mjc = (mjc < jc) ? jc : mjc;
             }
         }
@@ -600,412 +406,6 @@ __device__ __forceinline__ int tourn(int i1, int i2, const int32_t* rank, const 
     if (r2 < r1) return i2;
     if (__ldg(cd + i1) > __ldg(cd + i2)) return i1;
     return i2;
-}
-
-// residency target: 1280 threads per SM for one float4 group per thread, 1024 otherwise
-// (measured at n = 1000: 5 CTAs of 256 with 51 registers beat 6 with 40 and 8 with 32)
-template <int BLOCK, int G>
-struct RowResidency {
-    static constexpr int want = (G == 1 ? 1280 : 1024) / BLOCK;
-    static constexpr int value = want < 1 ? 1 : (want > 32 ? 32 : want);
-};
-
-template <int BLOCK, int G, bool DYN>
-__global__ void __launch_bounds__(BLOCK, RowResidency<BLOCK, G>::value) row_kernel(RowLaunch L) {
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    __shared__ PopDesc sd;
-    __shared__ uint32_t warp_tot[32];
-    __shared__ long long red_ll[64];
-    __shared__ float red_f[32];
-    __shared__ long long misc[4];
-
-    __shared__ int grab[2];
-
-    const int t = threadIdx.x;
-    const RowSmem s = carve(smem_raw, BLOCK, G, L.max_n, L.max_points);
-    int cur_pid = -1;
-    zero_counters<BLOCK, G>(s);
-    dep_wait();  // shared memory only above this line
-
-    // tasks are dealt to CTAs in groups of K consecutive tasks: neighbouring rows of one
-    // population stay in one CTA (its descriptor and coordinates are staged once per
-    // group).  Statically, group g goes to CTA g % grid.  With dynamic dealing (DYN, the
-    // shared launches of batches and the server, whose rows differ in length and kind), a
-    // CTA takes the next group from the work counter whenever it finishes one, so no SM
-    // idles while another still holds several long rows.
-    const int K = L.task_group > 1 ? L.task_group : 1;
-    if (DYN) {
-        if (t == 0) grab[0] = atomicAdd(L.work, K);
-        __syncthreads();
-    }
-    int round = 0;
-    for (int g0 = DYN ? grab[0] : blockIdx.x * K; g0 < L.ntasks;) {
-        int next = 0;
-        if (DYN && t == 0) next = atomicAdd(L.work, K);  // the following group, used after this one
-    for (int task = g0; task < min(L.ntasks, g0 + K); ++task) {
-        int pid = 0, r = task;
-        if (L.tasks) {
-            const Task tk = L.tasks[task];
-            pid = tk.pid;
-            r = tk.row;
-        }
-        if (pid != cur_pid) {
-            __syncthreads();
-            if (t == 0) sd = L.descs ? L.descs[pid] : L.single;
-            __syncthreads();
-            if (L.stage_xy && (sd.kind == TSP_COORDS || sd.kind == BITSP_COORDS)) {
-                const int npts = (sd.kind == BITSP_COORDS) ? sd.n + 1 : sd.n;
-                const float2* g0 = reinterpret_cast<const float2*>(sd.xy);
-                float2* d0 = reinterpret_cast<float2*>(s.xy);
-                for (int i = t; i < npts; i += BLOCK) d0[i] = g0[i];
-                if (sd.kind == BITSP_COORDS) {
-                    const float2* g1 = reinterpret_cast<const float2*>(sd.xy2);
-                    for (int i = t; i < npts; i += BLOCK) d0[npts + i] = g1[i];
-                }
-            }
-            __syncthreads();
-            cur_pid = pid;
-        }
-        const int n = sd.n, ld = sd.ld, P = sd.P, E = sd.E, M = sd.M, m = sd.m;
-        const int cur = sd.cur;
-        if ((L.mode == MODE_GEN || L.mode == MODE_NSGA_OFF) && at_limit(sd)) continue;
-        if (L.mode == MODE_NSGA_REFILL && !sd.advanced) continue;
-        if (!L.tasks && L.mode == MODE_GEN) r = (task < P - E) ? E + task : task - (P - E);
-        // local search: task = rank q; the row is the q-th best (the operator form works on
-        // rows in rank order already)
-        const int lsq = r;
-        if (L.mode == MODE_LSEARCH) {
-            if (!L.ls_force && (!ls_due(sd) || at_limit(sd))) continue;
-            if (!L.ls_force) r = __ldg(sd.sorted + lsq);
-        }
-
-        float k[G][4];
-        float* dst = nullptr;
-        float* dfit = nullptr;
-        bool eval = true, store = true;
-        const uint32_t isl = sd.island << 8;
-        // how the row is built: BUILD_LOAD (given keys), BUILD_COPY (elite), BUILD_RANDOM
-        // (fresh keys from one stream), BUILD_CROSS (biased crossover), BUILD_NSGA
-        // (uniform crossover + per-gene reset)
-        enum { BUILD_LOAD, BUILD_COPY, BUILD_RANDOM, BUILD_CROSS, BUILD_NSGA };
-        int build = BUILD_LOAD;
-        uint32_t gdraw = 0, tag0 = 0;
-        const float* src = sd.keys[cur];
-        int pa = 0, pb = 0;
-        if (L.mode == MODE_GEN) {
-            dst = sd.keys[cur ^ 1];
-            dfit = sd.fit[cur ^ 1];
-            gdraw = sd.gen + 1;
-            if (r < E) {
-                build = BUILD_COPY;
-            } else if (r < P - M) {
-                // biased crossover (core/solver.hpp:1109-1135; core/cuda_kernels.cuh:120-134)
-                build = BUILD_CROSS;
-                tag0 = isl | TAG_COIN;
-                int2 prk;
-                if (sd.parents) {
-                    prk = sd.parents[r];
-                } else {
-                    const uint4 pr = draw4(sd.seed, 0u, (uint32_t)r, gdraw, isl | TAG_PARENT);
-                    prk = make_int2((int)pick(pr.x, (uint32_t)E), E + (int)pick(pr.y, (uint32_t)(P - E)));
-                }
-                pa = __ldg(sd.sorted + prk.x);
-                pb = __ldg(sd.sorted + prk.y);
-            } else {
-                build = BUILD_RANDOM;  // mutant (core/solver.hpp:1244-1258)
-                tag0 = isl | TAG_MUTANT;
-            }
-        } else if (L.mode == MODE_INIT) {
-            // Population::initialize keys (core/population.hpp:107-110)
-            dst = sd.keys[cur];
-            dfit = sd.fit[cur];
-            build = BUILD_RANDOM;
-            tag0 = isl | TAG_INIT;
-        } else if (L.mode == MODE_NSGA_OFF) {
-            // NSGA-II offspring (core/solver.hpp:1019-1091): pool rows [P, 2P) of keys[cur]
-            dst = sd.keys[cur] + (size_t)P * ld;
-            dfit = sd.fit[cur] + (size_t)P * m;
-            gdraw = sd.gen + 1;
-            if (r >= P - sd.Mn) {
-                build = BUILD_RANDOM;
-                tag0 = TAG_MUTANT;
-            } else {
-                build = BUILD_NSGA;
-                tag0 = TAG_NSGA_COIN;
-                const uint4 pk = draw4(sd.seed, 0u, (uint32_t)r, gdraw, TAG_NSGA_TOUR);
-                pa = tourn(pick(pk.x, P), pick(pk.y, P), sd.nrank, sd.ncd);
-                pb = tourn(pick(pk.z, P), pick(pk.w, P), sd.nrank, sd.ncd);
-            }
-        } else if (L.mode == MODE_NSGA_REFILL) {
-            // ensure_minimum_diversity refill (core/population.hpp:166-171): rows from the
-            // unique count on are replaced by fresh random keys of generation sd.gen
-            if (r < __ldg(sd.nu)) continue;
-            dst = sd.keys[cur];
-            dfit = sd.fit[cur];
-            gdraw = sd.gen;
-            build = BUILD_RANDOM;
-            tag0 = TAG_NSGA_REFILL;
-        } else if (L.mode == MODE_LSEARCH) {
-            // random 2-opt (core/cuda_kernels.cuh:166-246): the row is rewritten in place, and
-            // only when the search improved it
-            dst = sd.keys[cur];
-            dfit = sd.fit[cur];
-            store = false;
-        } else {  // MODE_EVAL: given keys
-            dfit = sd.fit[cur];
-            store = false;
-        }
-
-        if (build == BUILD_COPY) {
-            // elite copy (core/population.hpp:700-714), fitness kept
-            const int sr = __ldg(sd.sorted + r);
-            const float4* a = reinterpret_cast<const float4*>(src + (size_t)sr * ld);
-            float4* o = reinterpret_cast<float4*>(dst + (size_t)r * ld);
-            for (int q = t; q < ld / 4; q += BLOCK) o[q] = __ldg(a + q);
-            if (t < m) dfit[(size_t)r * m + t] = __ldg(sd.fit[cur] + (size_t)sr * m + t);
-            eval = false;
-            store = false;
-        } else if (build == BUILD_LOAD) {
-            const float* row = src + (size_t)r * ld;
-            const bool vec = ((ld & 3) == 0) && ((reinterpret_cast<uintptr_t>(src) & 15) == 0);
-#pragma unroll
-            for (int gg = 0; gg < G; ++gg) {
-                const int q = t + gg * BLOCK;
-                if (vec && 4 * q + 3 < ld) {
-                    const float4 a = __ldg(reinterpret_cast<const float4*>(row) + q);
-                    k[gg][0] = a.x;
-                    k[gg][1] = a.y;
-                    k[gg][2] = a.z;
-                    k[gg][3] = a.w;
-                } else {
-#pragma unroll
-                    for (int l = 0; l < 4; ++l) k[gg][l] = (4 * q + l < n) ? __ldg(row + 4 * q + l) : 0.0f;
-                }
-            }
-        } else {
-            const float4* A = reinterpret_cast<const float4*>(src + (size_t)pa * ld);
-            const float4* Bv = reinterpret_cast<const float4*>(src + (size_t)pb * ld);
-#pragma unroll
-            for (int gg = 0; gg < G; ++gg) {
-                const int q = t + gg * BLOCK;
-                if (4 * q < n) {
-                    float4 a = make_float4(0.f, 0.f, 0.f, 0.f), b = a;
-                    if (build != BUILD_RANDOM) {
-                        a = __ldg(A + q);
-                        b = __ldg(Bv + q);
-                    }
-                    // one Philox call site per group for every way a row is built
-                    const uint4 x = draw4(sd.seed, (uint32_t)q, (uint32_t)r, gdraw, tag0);
-                    if (build == BUILD_RANDOM) {
-                        k[gg][0] = u24(x.x);
-                        k[gg][1] = u24(x.y);
-                        k[gg][2] = u24(x.z);
-                        k[gg][3] = u24(x.w);
-                    } else {
-                        const uint32_t T = sd.rhoT;
-                        k[gg][0] = ((x.x >> 8) < T) ? a.x : b.x;
-                        k[gg][1] = ((x.y >> 8) < T) ? a.y : b.y;
-                        k[gg][2] = ((x.z >> 8) < T) ? a.z : b.z;
-                        k[gg][3] = ((x.w >> 8) < T) ? a.w : b.w;
-                    }
-                    if (build == BUILD_NSGA) {
-                        const uint4 mp = draw4(sd.seed, (uint32_t)q, (uint32_t)r, gdraw, TAG_NSGA_MUTP);
-                        const uint4 mk = draw4(sd.seed, (uint32_t)q, (uint32_t)r, gdraw, TAG_NSGA_MUTK);
-                        const uint32_t T = sd.mutT;
-                        if ((mp.x >> 8) < T) k[gg][0] = u24(mk.x);
-                        if ((mp.y >> 8) < T) k[gg][1] = u24(mk.y);
-                        if ((mp.z >> 8) < T) k[gg][2] = u24(mk.z);
-                        if ((mp.w >> 8) < T) k[gg][3] = u24(mk.w);
-                    }
-                }
-            }
-        }
-
-        if (L.mode == MODE_LSEARCH) {
-            // reverse random segments [i, j] of the city keys (the first n/2 genes), as the
-            // reference's random_2opt_kernel: i, j uniform over the cities, ordered, skipped
-            // when j - i < 2; the composites buffer is free until the decode
-            const int c = n / 2;
-            float* sk = reinterpret_cast<float*>(s.sc);
-#pragma unroll
-            for (int gg = 0; gg < G; ++gg)
-#pragma unroll
-                for (int l = 0; l < 4; ++l) {
-                    const int i = 4 * (t + gg * BLOCK) + l;
-                    if (i < c) sk[i] = k[gg][l];
-                }
-            __syncthreads();
-            for (int mv = 0; mv < L.ls_moves; ++mv) {
-                const uint4 x = draw4(sd.seed, (uint32_t)mv, (uint32_t)lsq, sd.gen, isl | TAG_LS);
-                int i = (int)pick(x.x, (uint32_t)c), j = (int)pick(x.y, (uint32_t)c);
-                if (i > j) {
-                    const int tmp = i;
-                    i = j;
-                    j = tmp;
-                }
-                if (j - i >= 2)
-                    for (int p = t; p < (j - i + 1) / 2; p += BLOCK) {
-                        const float u = sk[i + p];
-                        sk[i + p] = sk[j - p];
-                        sk[j - p] = u;
-                    }
-                __syncthreads();
-            }
-#pragma unroll
-            for (int gg = 0; gg < G; ++gg)
-#pragma unroll
-                for (int l = 0; l < 4; ++l) {
-                    const int i = 4 * (t + gg * BLOCK) + l;
-                    if (i < c) k[gg][l] = sk[i];
-                }
-            __syncthreads();
-        }
-
-        if (store) {
-            // write the new row with 128-bit stores; padding lanes (>= n) are zero
-            float4* o = reinterpret_cast<float4*>(dst + (size_t)r * ld);
-#pragma unroll
-            for (int gg = 0; gg < G; ++gg) {
-                const int q = t + gg * BLOCK;
-                if (4 * q < ld) {
-                    float4 v;
-                    v.x = (4 * q + 0 < n) ? k[gg][0] : 0.0f;
-                    v.y = (4 * q + 1 < n) ? k[gg][1] : 0.0f;
-                    v.z = (4 * q + 2 < n) ? k[gg][2] : 0.0f;
-                    v.w = (4 * q + 3 < n) ? k[gg][3] : 0.0f;
-                    o[q] = v;
-                }
-            }
-        }
-
-        if (eval) {
-            float res[2] = {0.0f, 0.0f};
-            const int kind = sd.kind;
-            if (kind == KNAP_THRESHOLD) {
-                // configs/knapsack_config.hpp:43-62 (integer sums are exact as floats below 2^24)
-                long long tw = 0, tv = 0;
-#pragma unroll
-                for (int gg = 0; gg < G; ++gg)
-#pragma unroll
-                    for (int l = 0; l < 4; ++l) {
-                        const int i = 4 * (t + gg * BLOCK) + l;
-                        if (i < n && k[gg][l] > 0.5f) {
-                            tw += __ldg(sd.w + i);
-                            tv += __ldg(&sd.wv[i].y);
-                        }
-                    }
-                tw = block_sum_ll<BLOCK>(tw, red_ll);
-                tv = block_sum_ll<BLOCK>(tv, red_ll);
-                const float twf = (float)tw, tvf = (float)tv;
-                res[0] = (twf > sd.cap) ? __fsub_rn(tvf, __fmul_rn(__fsub_rn(twf, sd.cap), 1000.0f)) : tvf;
-            } else if (kind == CONTINUOUS || kind == JOBSCHED) {
-                // no decode: the keys in index order, staged where the sort composites go
-                float* sk = reinterpret_cast<float*>(s.sc);
-#pragma unroll
-                for (int gg = 0; gg < G; ++gg)
-#pragma unroll
-                    for (int l = 0; l < 4; ++l) {
-                        const int i = 4 * (t + gg * BLOCK) + l;
-                        if (i < n) sk[i] = k[gg][l];
-                    }
-                __syncthreads();
-                res[0] = (kind == CONTINUOUS) ? continuous_fitness<BLOCK>(sk, n, sd.function, sd.lo, sd.hi, red_f)
-                                              : jobsched_makespan<BLOCK>(sk, n, sd.jt, sd.machines, red_f);
-            } else {
-                row_argsort<BLOCK, G>(k, n, (kind == TSPJ) ? n / 2 : n, s, warp_tot);
-                zero_counters<BLOCK, G>(s);  // ready for the next row (separated by the row-end barrier)
-                const int32_t* perm = s.perm;
-                if (kind == TSP_COORDS) {
-                    const float* xy = L.stage_xy ? s.xy : sd.xy;
-                    canon_sum<BLOCK, 1>(n, [&](int e, float* d) {
-                        const int a = perm[e], b = perm[(e + 1 < n) ? e + 1 : 0];
-                        d[0] = edge_xy(xy, a, b);
-                    }, red_f, res);
-                } else if (kind == TSP_MATRIX) {
-                    const float* mat = sd.mat;
-                    canon_sum<BLOCK, 1>(n, [&](int e, float* d) {
-                        const int a = perm[e], b = perm[(e + 1 < n) ? e + 1 : 0];
-                        d[0] = __ldg(mat + (size_t)a * n + b);
-                    }, red_f, res);
-                } else if (kind == BITSP_COORDS) {
-                    const int npts = n + 1;
-                    const float* xy0 = L.stage_xy ? s.xy : sd.xy;
-                    const float* xy1 = L.stage_xy ? s.xy + 2 * npts : sd.xy2;
-                    canon_sum<BLOCK, 2>(n + 1, [&](int e, float* d) {
-                        const int a = (e == 0) ? 0 : perm[e - 1] + 1;
-                        const int b = (e == n) ? 0 : perm[e] + 1;
-                        d[0] = edge_xy(xy0, a, b);
-                        d[1] = edge_xy(xy1, a, b);
-                    }, red_f, res);
-                } else if (kind == BITSP_MATRIX) {
-                    const float* m0 = sd.mat;
-                    const float* m1 = sd.mat2;
-                    const size_t np1 = (size_t)n + 1;
-                    canon_sum<BLOCK, 2>(n + 1, [&](int e, float* d) {
-                        const int a = (e == 0) ? 0 : perm[e - 1] + 1;
-                        const int b = (e == n) ? 0 : perm[e] + 1;
-                        d[0] = __ldg(m0 + (size_t)a * np1 + b);
-                        d[1] = __ldg(m1 + (size_t)a * np1 + b);
-                    }, red_f, res);
-                } else if (kind == KNAP_GREEDY) {
-                    if constexpr (G == 1)
-                        res[0] = knap_greedy_call<BLOCK>(s.perm, n, sd.wv, sd.capi, red_ll, misc,
-                                                         reinterpret_cast<int2*>(s.sc));
-                    else
-                        res[0] = knap_greedy<BLOCK>(s.perm, n, sd.wv, sd.capi, red_ll, misc,
-                                                    reinterpret_cast<int2*>(s.sc));
-                } else if (kind == TSPJ) {
-                    if constexpr (G == 1)
-                        res[0] = tspj_makespan_call<BLOCK>(perm, n / 2, sd.mat, sd.mat2, red_f);
-                    else
-                        res[0] = tspj_makespan<BLOCK>(perm, n / 2, sd.mat, sd.mat2, red_f);
-                }
-                if (L.perm_out) {
-                    int32_t* po = L.perm_out + (size_t)r * n;
-                    for (int i = t; i < n; i += BLOCK) po[i] = perm[i];
-                }
-            }
-            if (L.mode == MODE_LSEARCH) {
-                // keep the searched row only if it is better (restore_if_worse_kernel)
-                const float old = dfit[(size_t)r * m];
-                if (sd.maximize ? (res[0] > old) : (res[0] < old)) {
-                    __syncthreads();  // every thread has read the old value
-                    float4* o = reinterpret_cast<float4*>(dst + (size_t)r * ld);
-#pragma unroll
-                    for (int gg = 0; gg < G; ++gg) {
-                        const int q = t + gg * BLOCK;
-                        if (4 * q < ld) {
-                            float4 v;
-                            v.x = (4 * q + 0 < n) ? k[gg][0] : 0.0f;
-                            v.y = (4 * q + 1 < n) ? k[gg][1] : 0.0f;
-                            v.z = (4 * q + 2 < n) ? k[gg][2] : 0.0f;
-                            v.w = (4 * q + 3 < n) ? k[gg][3] : 0.0f;
-                            o[q] = v;
-                        }
-                    }
-                    if (t == 0) dfit[(size_t)r * m] = res[0];
-                }
-            } else {
-                if (t == 0) dfit[(size_t)r * m] = res[0];
-                if (t == 1 && m > 1) dfit[(size_t)r * m + 1] = res[1];
-            }
-        }
-        __syncthreads();
-    }
-        if (DYN) {
-            ++round;
-            if (t == 0) grab[round & 1] = next;
-            __syncthreads();
-            g0 = grab[round & 1];
-        } else {
-            g0 += gridDim.x * K;
-        }
-    }
-    if (DYN && t == 0 && atomicAdd(L.work + 1, 1) == (int)gridDim.x - 1) {
-        // every CTA has taken its last group: leave the counter zero for the next launch
-        L.work[0] = 0;
-        L.work[1] = 0;
-    }
 }
 
 // ---------------------------------------------------------------------------------------
@@ -1441,317 +841,6 @@ __global__ void migrate_kernel(PopDesc* descs, int k, int mig) {
 }
 
 // ---------------------------------------------------------------------------------------
-// MO-VRP rows (MultiObjectiveVRPConfig, configs/multi_objective_vrp_config.hpp).  A kernel of
-// their own, so the other kinds' row kernel keeps its registers: it builds rows exactly as
-// the row kernel does in the modes an NSGA-II population uses (initial keys, offspring,
-// diversity refill, given keys), then decodes and scores them:
-//   1. h = the FP32 sum of key_i * (i + 1) in index order (one warp, keys staged in shared
-//      memory); the sort value of gene i is key_i + (i * 1e-5 + h * 1e-5)  (:219-230);
-//   2. a stable argsort of the values, ties to the lower index (std::sort over (value,
-//      customer) pairs);
-//   3. one warp walks the order, closing a route when the next demand would take a
-//      non-empty route over capacity, and forms both objectives with the overload and
-//      fleet penalties in the reference's order of float additions (:233-313).
-// ---------------------------------------------------------------------------------------
-
-// the bucket argsort of row_argsort with buckets over (value - lo) * inv, lo = h * 1e-5 and
-// inv = 1 / (1 + n * 1e-5): the values span about [lo, lo + 1 + n * 1e-5], and any
-// non-decreasing bucket map gives the same (value, index) order
-template <int BLOCK, int G>
-__device__ void movrp_argsort(const float (&v)[G][4], int n, float lo, float inv, const RowSmem& s,
-                              uint32_t* warp_tot) {
-    constexpr int NB = 4 * G * BLOCK;
-    const int t = threadIdx.x;
-    uint32_t bs[G][4];
-#pragma unroll
-    for (int g = 0; g < G; ++g)
-#pragma unroll
-        for (int l = 0; l < 4; ++l) {
-            const int i = 4 * (t + g * BLOCK) + l;
-            if (i < n) {
-                const int b = bucket_of(__fmul_rn(__fsub_rn(v[g][l], lo), inv), (float)NB, NB);
-                bs[g][l] = ((uint32_t)b << 16) | atomicAdd(&s.cnt[b], 1u);
-            }
-        }
-    __syncthreads();
-    uint4 c[G];
-    uint32_t sum = 0, big = 0;
-#pragma unroll
-    for (int g = 0; g < G; ++g) {
-        c[g] = reinterpret_cast<const uint4*>(s.cnt)[t * G + g];
-        sum += c[g].x + c[g].y + c[g].z + c[g].w;
-        big = max(big, max(max(c[g].x, c[g].y), max(c[g].z, c[g].w)));
-    }
-    uint32_t run = block_exclusive_scan<BLOCK>(sum, warp_tot, nullptr);
-#pragma unroll
-    for (int g = 0; g < G; ++g) {
-        const uint4 o = make_uint4(run, run + c[g].x, run + c[g].x + c[g].y, run + c[g].x + c[g].y + c[g].z);
-        run = o.w + c[g].w;
-        reinterpret_cast<uint4*>(s.cnt)[t * G + g] = o;
-    }
-    if (t == 0) s.cnt[NB] = (uint32_t)n;
-    const bool heavy = __syncthreads_or(big > kHeavyBucket) != 0;
-#pragma unroll
-    for (int g = 0; g < G; ++g)
-#pragma unroll
-        for (int l = 0; l < 4; ++l) {
-            const int i = 4 * (t + g * BLOCK) + l;
-            if (i < n)
-                s.sc[s.cnt[bs[g][l] >> 16] + (bs[g][l] & 0xFFFFu)] =
-                    ((unsigned long long)okey(v[g][l]) << 32) | (uint32_t)i;
-        }
-    __syncthreads();
-    if (heavy) {  // equal or extreme values in few buckets: sort the composites instead
-        heavy_row_perm<BLOCK>(s.sc, s.perm, n, n);
-        return;
-    }
-#pragma unroll
-    for (int g = 0; g < G; ++g)
-#pragma unroll
-        for (int l = 0; l < 4; ++l) {
-            const int i = 4 * (t + g * BLOCK) + l;
-            if (i < n) {
-                const uint32_t b = bs[g][l] >> 16, b0 = s.cnt[b], b1 = s.cnt[b + 1];
-                const unsigned long long me = ((unsigned long long)okey(v[g][l]) << 32) | (uint32_t)i;
-                uint32_t r = b0;
-                for (uint32_t q = b0; q < b1; ++q) r += (s.sc[q] < me) ? 1u : 0u;
-                s.perm[r] = i;
-            }
-        }
-    __syncthreads();
-}
-
-// routes and objectives of the sorted customers perm[j] + 1.  Lanes fetch the legs (from the
-// previous customer, and to the depot) and demands of 128 positions at a time, loads first;
-// every lane then replays them in order, so all lanes hold the same state.  d(a, b) = d(b, a)
-// bit for bit (dx and -dx have the same square), so the depot leg into a route's first
-// customer is its leg to the depot.
-__device__ void movrp_objectives(const int32_t* perm, int n, const float* __restrict__ xy,
-                                 const int32_t* __restrict__ dem, int cap, int vehicles, float* red, float* out) {
-    constexpr int kChunks = 4;
-    if (threadIdx.x < 32) {
-        const int lane = threadIdx.x;
-        float dist = 0.0f, total = 0.0f, longest = 0.0f, pen = 0.0f, lastdep = 0.0f;
-        int load = 0, size = 0, routes = 0;
-        for (int g0 = 0; g0 < n; g0 += 32 * kChunks) {
-            float e[kChunks], dep[kChunks];
-            int dm[kChunks];
-#pragma unroll
-            for (int c = 0; c < kChunks; ++c) {
-                const int j = g0 + 32 * c + lane;
-                e[c] = 0.0f;
-                dep[c] = 0.0f;
-                dm[c] = 0;
-                if (j < n) {
-                    const int cust = perm[j] + 1;
-                    e[c] = edge_xy(xy, (j == 0) ? 0 : perm[j - 1] + 1, cust);
-                    dep[c] = edge_xy(xy, cust, 0);
-                    dm[c] = __ldg(dem + cust);
-                }
-            }
-#pragma unroll
-            for (int c = 0; c < kChunks; ++c) {
-                const int cnt = min(32, n - (g0 + 32 * c));
-                for (int q = 0; q < cnt; ++q) {
-                    const float eq = __shfl_sync(0xffffffffu, e[c], q);
-                    const float dq = __shfl_sync(0xffffffffu, dep[c], q);
-                    const int mq = __shfl_sync(0xffffffffu, dm[c], q);
-                    if (load + mq > cap && size > 0) {  // close the route: back to the depot
-                        dist = __fadd_rn(dist, lastdep);
-                        total = __fadd_rn(total, dist);
-                        longest = (dist > longest) ? dist : longest;
-                        if (load > cap) pen = __fadd_rn(pen, __fmul_rn((float)(load - cap), 100.0f));
-                        ++routes;
-                        dist = 0.0f;
-                        load = 0;
-                        size = 0;
-                    }
-                    dist = __fadd_rn(dist, (size == 0) ? dq : eq);
-                    load += mq;
-                    ++size;
-                    lastdep = dq;
-                }
-            }
-        }
-        if (size > 0) {
-            dist = __fadd_rn(dist, lastdep);
-            total = __fadd_rn(total, dist);
-            longest = (dist > longest) ? dist : longest;
-            if (load > cap) pen = __fadd_rn(pen, __fmul_rn((float)(load - cap), 100.0f));
-            ++routes;
-        }
-        float o0 = __fadd_rn(total, pen), o1 = longest;
-        if (routes > vehicles) {
-            const float vp = __fmul_rn((float)(routes - vehicles), 500.0f);
-            o0 = __fadd_rn(o0, vp);
-            o1 = __fadd_rn(o1, vp);
-        }
-        if (lane == 0) {
-            red[0] = o0;
-            red[1] = o1;
-        }
-    }
-    __syncthreads();
-    out[0] = red[0];
-    out[1] = red[1];
-    __syncthreads();
-}
-
-template <int BLOCK, int G>
-__global__ void __launch_bounds__(BLOCK, RowResidency<BLOCK, G>::value) movrp_row_kernel(RowLaunch L) {
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    __shared__ PopDesc sd;
-    __shared__ uint32_t warp_tot[32];
-    __shared__ float red_f[32];
-    const int t = threadIdx.x;
-    const RowSmem s = carve(smem_raw, BLOCK, G, L.max_n, L.max_points);
-    int cur_pid = -1;
-    zero_counters<BLOCK, G>(s);
-    dep_wait();  // shared memory only above this line
-
-    for (int task = blockIdx.x; task < L.ntasks; task += gridDim.x) {
-        int pid = 0, r = task;
-        if (L.tasks) {
-            const Task tk = L.tasks[task];
-            pid = tk.pid;
-            r = tk.row;
-        }
-        if (pid != cur_pid) {
-            __syncthreads();
-            if (t == 0) sd = L.descs ? L.descs[pid] : L.single;
-            __syncthreads();
-            cur_pid = pid;
-        }
-        const int n = sd.n, ld = sd.ld, P = sd.P, m = sd.m, cur = sd.cur;
-        if (L.mode == MODE_NSGA_OFF && at_limit(sd)) continue;
-        if (L.mode == MODE_NSGA_REFILL && (!sd.advanced || r < __ldg(sd.nu))) continue;
-        const float* src = sd.keys[cur];
-        float* dst = nullptr;
-        float* dfit = nullptr;
-        enum { LOAD, RANDOM, NSGA } build = RANDOM;
-        uint32_t gdraw = 0, tag = 0;
-        int pa = 0, pb = 0;
-        if (L.mode == MODE_INIT) {  // core/population.hpp:107-110
-            dst = sd.keys[cur];
-            dfit = sd.fit[cur];
-            tag = (sd.island << 8) | TAG_INIT;
-        } else if (L.mode == MODE_NSGA_OFF) {  // core/solver.hpp:1019-1091, pool rows [P, 2P)
-            dst = sd.keys[cur] + (size_t)P * ld;
-            dfit = sd.fit[cur] + (size_t)P * m;
-            gdraw = sd.gen + 1;
-            if (r >= P - sd.Mn) {
-                tag = TAG_MUTANT;
-            } else {
-                build = NSGA;
-                tag = TAG_NSGA_COIN;
-                const uint4 pk = draw4(sd.seed, 0u, (uint32_t)r, gdraw, TAG_NSGA_TOUR);
-                pa = tourn(pick(pk.x, P), pick(pk.y, P), sd.nrank, sd.ncd);
-                pb = tourn(pick(pk.z, P), pick(pk.w, P), sd.nrank, sd.ncd);
-            }
-        } else if (L.mode == MODE_NSGA_REFILL) {  // core/population.hpp:166-171
-            dst = sd.keys[cur];
-            dfit = sd.fit[cur];
-            gdraw = sd.gen;
-            tag = TAG_NSGA_REFILL;
-        } else if (L.mode == MODE_EVAL) {
-            dfit = sd.fit[cur];
-            build = LOAD;
-        } else {
-            continue;  // single-objective modes do not apply
-        }
-
-        float k[G][4];
-        const float* row = src + (size_t)r * ld;
-        const bool vec = ((ld & 3) == 0) && ((reinterpret_cast<uintptr_t>(src) & 15) == 0);
-#pragma unroll
-        for (int gg = 0; gg < G; ++gg) {
-            const int q = t + gg * BLOCK;
-#pragma unroll
-            for (int l = 0; l < 4; ++l) k[gg][l] = 0.0f;
-            if (build == LOAD) {
-                if (vec && 4 * q + 3 < ld) {
-                    const float4 a = __ldg(reinterpret_cast<const float4*>(row) + q);
-                    k[gg][0] = a.x, k[gg][1] = a.y, k[gg][2] = a.z, k[gg][3] = a.w;
-                } else {
-#pragma unroll
-                    for (int l = 0; l < 4; ++l) k[gg][l] = (4 * q + l < n) ? __ldg(row + 4 * q + l) : 0.0f;
-                }
-            } else if (4 * q < n) {
-                const uint4 x = draw4(sd.seed, (uint32_t)q, (uint32_t)r, gdraw, tag);
-                if (build == RANDOM) {
-                    k[gg][0] = u24(x.x), k[gg][1] = u24(x.y), k[gg][2] = u24(x.z), k[gg][3] = u24(x.w);
-                } else {
-                    const float4 a = __ldg(reinterpret_cast<const float4*>(src + (size_t)pa * ld) + q);
-                    const float4 b = __ldg(reinterpret_cast<const float4*>(src + (size_t)pb * ld) + q);
-                    const uint32_t T = sd.rhoT, MT = sd.mutT;
-                    k[gg][0] = ((x.x >> 8) < T) ? a.x : b.x;
-                    k[gg][1] = ((x.y >> 8) < T) ? a.y : b.y;
-                    k[gg][2] = ((x.z >> 8) < T) ? a.z : b.z;
-                    k[gg][3] = ((x.w >> 8) < T) ? a.w : b.w;
-                    const uint4 mp = draw4(sd.seed, (uint32_t)q, (uint32_t)r, gdraw, TAG_NSGA_MUTP);
-                    const uint4 mk = draw4(sd.seed, (uint32_t)q, (uint32_t)r, gdraw, TAG_NSGA_MUTK);
-                    if ((mp.x >> 8) < MT) k[gg][0] = u24(mk.x);
-                    if ((mp.y >> 8) < MT) k[gg][1] = u24(mk.y);
-                    if ((mp.z >> 8) < MT) k[gg][2] = u24(mk.z);
-                    if ((mp.w >> 8) < MT) k[gg][3] = u24(mk.w);
-                }
-            }
-            if (build != LOAD && 4 * q < ld) {
-                float4 o;
-                o.x = (4 * q + 0 < n) ? k[gg][0] : 0.0f;
-                o.y = (4 * q + 1 < n) ? k[gg][1] : 0.0f;
-                o.z = (4 * q + 2 < n) ? k[gg][2] : 0.0f;
-                o.w = (4 * q + 3 < n) ? k[gg][3] : 0.0f;
-                reinterpret_cast<float4*>(dst + (size_t)r * ld)[q] = o;
-            }
-        }
-
-        // 1. the row hash and the sort values
-        float* sk = reinterpret_cast<float*>(s.sc);
-#pragma unroll
-        for (int gg = 0; gg < G; ++gg)
-#pragma unroll
-            for (int l = 0; l < 4; ++l) {
-                const int i = 4 * (t + gg * BLOCK) + l;
-                if (i < n) sk[i] = k[gg][l];
-            }
-        __syncthreads();
-        if (t < 32) {
-            float h = 0.0f;
-            for (int c0 = 0; c0 < n; c0 += 32) {
-                const int i = c0 + t;
-                const float term = (i < n) ? __fmul_rn(sk[i], (float)(i + 1)) : 0.0f;
-                const int cnt = min(32, n - c0);
-                for (int q = 0; q < cnt; ++q) h = __fadd_rn(h, __shfl_sync(0xffffffffu, term, q));
-            }
-            if (t == 0) red_f[0] = h;
-        }
-        __syncthreads();
-        const float hb = __fmul_rn(red_f[0], 1.0e-5f);
-#pragma unroll
-        for (int gg = 0; gg < G; ++gg)
-#pragma unroll
-            for (int l = 0; l < 4; ++l) {
-                const int i = 4 * (t + gg * BLOCK) + l;
-                k[gg][l] = (i < n) ? __fadd_rn(k[gg][l], __fadd_rn(__fmul_rn((float)i, 1.0e-5f), hb)) : 0.0f;
-            }
-        __syncthreads();  // red_f[0] and the staged keys are read
-        // 2. the visiting order
-        movrp_argsort<BLOCK, G>(k, n, hb, __frcp_rn(__fadd_rn(1.0f, __fmul_rn((float)n, 1.0e-5f))), s, warp_tot);
-        zero_counters<BLOCK, G>(s);  // ready for the next row (separated by the row-end barrier)
-        // 3. routes and objectives
-        float res[2];
-        movrp_objectives(s.perm, n, sd.xy, sd.w, (int)sd.capi, sd.machines, red_f, res);
-        if (L.perm_out) {
-            int32_t* po = L.perm_out + (size_t)r * n;
-            for (int i = t; i < n; i += BLOCK) po[i] = s.perm[i];
-        }
-        if (t < 2) dfit[(size_t)r * m + t] = res[t];
-        __syncthreads();
-    }
-}
-
-// ---------------------------------------------------------------------------------------
 // host side
 // ---------------------------------------------------------------------------------------
 int device_sm_count() {
@@ -1761,42 +850,6 @@ int device_sm_count() {
     return sms;
 }
 
-// default tile per size (smallest capacity 4 * block * groups that covers n); the
-// autotuner may pick any other tile whose capacity covers n
-static constexpr RowTile kTiles[] = {
-    {32, 1}, {64, 1}, {128, 1}, {256, 1}, {256, 2}, {512, 2}, {512, 4}, {1024, 3}, {1024, 4},
-};
-static constexpr RowTile kAllTiles[] = {
-    {32, 1}, {64, 1}, {64, 2}, {128, 1}, {128, 2}, {128, 4}, {256, 1}, {256, 2}, {256, 4},
-    {512, 1}, {512, 2}, {512, 4}, {1024, 1}, {1024, 2}, {1024, 3}, {1024, 4},
-};
-
-int tile_candidates(int n, RowTile* out, int cap) {
-    int c = 0;
-    for (const RowTile& t : kAllTiles)
-        if (4 * t.block * t.groups >= n && 4 * t.block * t.groups <= 8 * n + 128 && c < cap) out[c++] = t;
-    return c;
-}
-
-RowTile pick_tile(int n) {
-    for (const RowTile& t : kTiles)
-        if (4 * t.block * t.groups >= n) return t;
-    return RowTile{0, 0};
-}
-
-int row_max_n() { return 4 * 1024 * 4; }
-
-int row_max_n_global() { return 1 << 22; }
-
-bool row_needs_global(int n, int pts, int kind) {
-    // rows of an external-fitness problem are only built: the global kernel builds them
-    // without a sort buffer in shared memory
-    if (kind == EXTERNAL) return true;
-    if (n > row_max_n()) return true;
-    const RowTile t = pick_tile(n);
-    return row_smem_bytes(t, n, pts, kind, false) > kRowSmemCap;
-}
-
 int row_global_grid(int rows, int max_n) {
     const size_t budget = (size_t)2 << 30;  // scratch for at most 2 GiB of CTAs
     int g = 2 * device_sm_count();
@@ -1804,54 +857,6 @@ int row_global_grid(int rows, int max_n) {
     if ((size_t)g > by_mem) g = (int)by_mem;
     if (g > rows) g = rows;
     return g < 1 ? 1 : g;
-}
-
-using RowFn = void (*)(RowLaunch);
-
-static RowFn row_fn(const RowTile& t, bool dyn = false) {
-#define BK_TILE(B, G) \
-    if (t.block == B && t.groups == G) return dyn ? row_kernel<B, G, true> : row_kernel<B, G, false>;
-    BK_TILE(32, 1)
-    BK_TILE(64, 1)
-    BK_TILE(64, 2)
-    BK_TILE(128, 1)
-    BK_TILE(128, 2)
-    BK_TILE(128, 4)
-    BK_TILE(256, 1)
-    BK_TILE(256, 2)
-    BK_TILE(256, 4)
-    BK_TILE(512, 1)
-    BK_TILE(512, 2)
-    BK_TILE(512, 4)
-    BK_TILE(1024, 1)
-    BK_TILE(1024, 2)
-    BK_TILE(1024, 3)
-    BK_TILE(1024, 4)
-#undef BK_TILE
-    return nullptr;
-}
-
-static RowFn movrp_fn(const RowTile& t) {
-#define BK_TILE(B, G) \
-    if (t.block == B && t.groups == G) return movrp_row_kernel<B, G>;
-    BK_TILE(32, 1)
-    BK_TILE(64, 1)
-    BK_TILE(64, 2)
-    BK_TILE(128, 1)
-    BK_TILE(128, 2)
-    BK_TILE(128, 4)
-    BK_TILE(256, 1)
-    BK_TILE(256, 2)
-    BK_TILE(256, 4)
-    BK_TILE(512, 1)
-    BK_TILE(512, 2)
-    BK_TILE(512, 4)
-    BK_TILE(1024, 1)
-    BK_TILE(1024, 2)
-    BK_TILE(1024, 3)
-    BK_TILE(1024, 4)
-#undef BK_TILE
-    return nullptr;
 }
 
 // the dynamic shared-memory limit of a kernel is only ever raised, so a later launch
@@ -1870,41 +875,14 @@ cudaError_t raise_smem_limit(const void* fn, size_t smem) {
     return e;
 }
 
-cudaError_t prepare_rows(const RowTile& tile, size_t smem, int* per_sm) {
-    RowFn fn = row_fn(tile);
-    if (!fn) return cudaErrorInvalidValue;
-    cudaError_t e = raise_smem_limit(reinterpret_cast<const void*>(fn), smem);
-    if (e == cudaSuccess) e = raise_smem_limit(reinterpret_cast<const void*>(row_fn(tile, true)), smem);
-    // the MO-VRP kernel has the same launch bounds and shared memory
-    if (e == cudaSuccess) e = raise_smem_limit(reinterpret_cast<const void*>(movrp_fn(tile)), smem);
-    if (e != cudaSuccess) return e;
-    return cudaOccupancyMaxActiveBlocksPerMultiprocessor(per_sm, fn, tile.block, smem);
-}
-
-cudaError_t launch_rows(const RowLaunch& L, int kind, const RowTile& tile, int grid, cudaStream_t s) {
-    if (tile.block == 0) {  // rows beyond shared memory: global-scratch kernel
-        if (!L.gscratch || L.gstride < row_global_stride(L.max_n)) return cudaErrorInvalidValue;
-        if (kind == MOVRP) return cudaErrorInvalidValue;  // MO-VRP rows fit in shared memory only
-        if (L.ntasks <= 0 || grid <= 0) return cudaSuccess;
-        if (grid > L.ntasks) grid = L.ntasks;
-        row_kernel_big<<<grid, kBigBlock, 0, s>>>(L);
-        return cudaGetLastError();
-    }
-    RowFn fn = (kind == MOVRP) ? movrp_fn(tile) : row_fn(tile, L.work != nullptr);
-    if (!fn) return cudaErrorInvalidValue;
+// rows beyond shared memory
+cudaError_t launch_rows_global(const RowLaunch& L, int kind, int grid, cudaStream_t s) {
+    if (!L.gscratch || L.gstride < row_global_stride(L.max_n)) return cudaErrorInvalidValue;
+    if (kind == MOVRP) return cudaErrorInvalidValue;  // MO-VRP rows fit in shared memory only
     if (L.ntasks <= 0 || grid <= 0) return cudaSuccess;
     if (grid > L.ntasks) grid = L.ntasks;
-    const size_t smem = row_smem_bytes(tile, L.max_n, L.max_points, kind, L.stage_xy != 0);
-    return launch_dep(fn, dim3(grid), dim3(tile.block), smem, s, L);
-}
-
-cudaError_t launch_rows_auto(const RowLaunch& L, int kind, const RowTile& tile, cudaStream_t s) {
-    const size_t smem = row_smem_bytes(tile, L.max_n, L.max_points, kind, L.stage_xy != 0);
-    int per_sm = 0;
-    cudaError_t e = prepare_rows(tile, smem, &per_sm);
-    if (e != cudaSuccess) return e;
-    if (per_sm <= 0) return cudaErrorInvalidConfiguration;
-    return launch_rows(L, kind, tile, per_sm * device_sm_count(), s);
+    row_kernel_big<<<grid, kBigBlock, 0, s>>>(L);
+    return cudaGetLastError();
 }
 
 cudaError_t prepare_sort(int maxP) {

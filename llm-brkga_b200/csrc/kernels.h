@@ -17,6 +17,17 @@ enum Mode : int32_t {
     MODE_LSEARCH = 5,  // TSPJ random 2-opt on the top ranks (task = rank)
 };
 
+// classes of kinds with a row kernel each: one-objective tours and the greedy knapsack (an
+// argsort and a sum), TSPJ (two argsorts), MO-VRP (an argsort of derived values), fitness
+// straight from the keys, the bi-objective TSP (NSGA-II builds, two tours)
+enum RowClass : int32_t { ROWS_ORDER = 0, ROWS_TSPJ = 1, ROWS_MOVRP = 2, ROWS_KEYS = 3, ROWS_BITSP = 4 };
+inline int row_class(int kind) {
+    if (kind == TSPJ) return ROWS_TSPJ;
+    if (kind == MOVRP) return ROWS_MOVRP;
+    if (kind == BITSP_COORDS || kind == BITSP_MATRIX) return ROWS_BITSP;
+    return (kind == KNAP_THRESHOLD || kind == JOBSCHED || kind == CONTINUOUS) ? ROWS_KEYS : ROWS_ORDER;
+}
+
 // one unit of row work: population `pid`, row `row` of that population
 struct Task {
     int32_t pid;
@@ -36,12 +47,14 @@ struct RowLaunch {
     int32_t ntasks;
     int32_t mode;
     int32_t* perm_out;       // optional decoded permutations [rows][n] (MODE_EVAL)
+    int32_t groups_per_cta;  // row groups per CTA (0, 1: one)
+    int32_t keep_keys;       // rows keep their keys in shared memory (set by launch_rows)
     int32_t max_n;           // largest chromosome among the populations launched
     int32_t max_points;      // largest coordinate count (n, or n+1 with a depot)
     int32_t stage_xy;        // stage coordinates in shared memory
     void* gscratch;          // global-scratch kernel (RowTile{0,0}): grid slices of gstride bytes
     size_t gstride;
-    int32_t task_group;      // tasks dealt to CTAs in groups of this many consecutive tasks (0, 1: one)
+    int32_t task_group;      // with a task list: tasks dealt to CTAs in units of this many (0, 1: one; <= 32)
     int32_t* work;           // dynamic dealing (batches and the server): [next group, CTAs done],
                              // zero before the launch and left zero by its last CTA; nullptr:
                              // group g goes to CTA g % grid
@@ -54,7 +67,11 @@ RowTile pick_tile(int n);
 // every compiled tile whose capacity covers n without being far larger (autotuning set)
 int tile_candidates(int n, RowTile* out, int cap);
 // shared memory bytes for one CTA of the row kernel
-size_t row_smem_bytes(const RowTile& t, int max_n, int max_points, int kind, bool stage_xy);
+size_t row_smem_bytes(const RowTile& t, int max_n, int max_points, int kind, bool stage_xy, int groups_per_cta);
+// row groups a CTA of this tile holds in a launch over many populations of mixed sizes
+int row_groups_shared(const RowTile& t, int max_n, int max_points, int kind, bool stage_xy);
+// row groups a CTA of this tile holds when a launch over one instance has `rows` rows
+int row_groups_per_cta(const RowTile& t, int max_n, int max_points, int kind, bool stage_xy, int rows);
 // largest n the in-shared-memory row kernel supports
 int row_max_n();
 // Rows whose sort does not fit in shared memory are decoded by a kernel with its sort
@@ -67,10 +84,12 @@ size_t row_global_stride(int max_n);
 int row_global_grid(int rows, int max_n);
 // one-time set-up for a tile / shared-memory size: raises the dynamic shared-memory limit
 // and returns the resident CTAs per SM (0 if the tile cannot run with that much memory)
-cudaError_t prepare_rows(const RowTile& tile, size_t smem, int* per_sm);
+cudaError_t prepare_rows(const RowTile& tile, int kind, int groups_per_cta, size_t smem, int* per_sm);
 // launch the fused row kernel (generation / init / evaluate / NSGA-II offspring) on
 // `grid` CTAs (<= resident capacity); prepare_rows must have run for this tile and size
 cudaError_t launch_rows(const RowLaunch& L, int kind, const RowTile& tile, int grid, cudaStream_t s);
+// the same for rows whose sort does not fit in shared memory (kGlobalTile)
+cudaError_t launch_rows_global(const RowLaunch& L, int kind, int grid, cudaStream_t s);
 // convenience for one-off launches: prepare + launch with an occupancy-sized grid
 cudaError_t launch_rows_auto(const RowLaunch& L, int kind, const RowTile& tile, cudaStream_t s);
 // raise the shared-memory limit of the sort kernels for populations of up to maxP rows

@@ -1600,7 +1600,7 @@ int32_t nsga_alloc(PopDesc& d, int P, double mut_rate, int div_interval, int Mn,
 }
 
 int32_t nsga_setup(NsgaState& s, Population& pop, PopDesc* dd, PopDesc& hdesc, const RowTile& tile, int grid,
-                   bool stage) {
+                   int groups_per_cta, bool stage) {
     s.dd = dd;
     s.P = pop.sh.Pi;
     s.N = 2 * pop.sh.Pi;
@@ -1612,6 +1612,7 @@ int32_t nsga_setup(NsgaState& s, Population& pop, PopDesc* dd, PopDesc& hdesc, c
     s.max_points = points_of(*pop.pd);
     s.tile = tile;
     s.grid = grid;
+    s.groups_per_cta = groups_per_cta;
     s.stage = stage;
     const double rate = (pop.prm.mutation_rate > 0.0) ? pop.prm.mutation_rate : 5.0 / (double)pop.sh.n;
     int32_t st = nsga_alloc(hdesc, s.P, rate, pop.prm.diversity_interval, pop.sh.Mn, pop.allocs, &pop.bytes,
@@ -1643,6 +1644,7 @@ static RowLaunch nsga_rows(const NsgaState& s, int mode) {
     L.max_n = s.n;
     L.max_points = s.max_points;
     L.stage_xy = s.stage ? 1 : 0;
+    L.groups_per_cta = s.groups_per_cta;
     L.gscratch = s.gscratch;
     L.gstride = s.gstride;
     return L;

@@ -15,7 +15,7 @@ struct NsgaState {
     PopDesc* dd = nullptr;   // device descriptor of the population (buffers live in it)
     int P = 0, N = 0, n = 0, ld = 0, kind = 0, max_points = 0;
     RowTile tile{};
-    int grid = 0;
+    int grid = 0, groups_per_cta = 1;
     bool stage = false;
     float* history = nullptr;
     int hist_cap = 0;
@@ -26,7 +26,7 @@ struct NsgaState {
 };
 
 int32_t nsga_setup(NsgaState& s, Population& pop, PopDesc* dd, PopDesc& hdesc, const RowTile& tile, int grid,
-                   bool stage);
+                   int groups_per_cta, bool stage);
 // allocate one population's NSGA-II buffers and fill its descriptor fields
 int32_t nsga_alloc(PopDesc& d, int P, double mut_rate, int div_interval, int Mn, std::vector<void*>& allocs,
                    size_t* bytes, cudaStream_t stream);
