@@ -368,7 +368,7 @@ namespace bk {
 // stream-ordered pool and returned to it behind the launch.
 static cudaError_t launch_op_rows(RowLaunch& L, const ProblemData& pd, cudaStream_t st) {
     if (!row_needs_global(pd.n, points_of(pd), pd.kind)) {
-        const RowTile tile = pick_tile(pd.n);
+        const RowTile tile = pick_tile(pd.n, pd.kind);
         L.stage_xy = stage_fits(tile, pd.n, L.max_points, pd.kind) ? 1 : 0;
         return launch_rows_auto(L, pd.kind, tile, st);
     }

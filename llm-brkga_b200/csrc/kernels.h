@@ -62,8 +62,8 @@ struct RowLaunch {
     int32_t ls_force;        // MODE_LSEARCH: run whatever the generation (operator); rank q = row q
 };
 
-// smallest tile whose capacity (4 * block * groups) covers n
-RowTile pick_tile(int n);
+// the default tile for rows of n keys
+RowTile pick_tile(int n, int kind);
 // every compiled tile whose capacity covers n without being far larger (autotuning set)
 int tile_candidates(int n, RowTile* out, int cap);
 // shared memory bytes for one CTA of the row kernel

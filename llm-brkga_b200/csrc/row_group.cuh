@@ -674,33 +674,42 @@ __device__ __forceinline__ float continuous_fitness(int n, int fn, float lo, flo
 // machine (int)(key_i * machines), capped at machines - 1; each machine's load adds its jobs
 // in index order; the makespan is the largest load.  The machines of all jobs are staged as
 // integers over s.sk; a thread keeps up to NM machines and passes all jobs in order, four
-// per 128-bit load (every lane of a warp reads the same four): a compare and a predicated
+// per 128-bit load (every lane of a warp reads the same four): a compare, a select and an
 // addition per machine and job, so each load equals the reference's sequential sum bit for
 // bit.  Handing the jobs round by two shuffles each took 60 us at n = 1000, 32 machines,
 // P = 2048.
 template <int T, int NM>
-__device__ __forceinline__ float jobsched_pass(const int32_t* mid, int n, const float* __restrict__ jt, int M, int m0) {
+__device__ __forceinline__ float jobsched_pass(const int32_t* mid, int n, const float* jt, int M, int m0) {
     float load[NM];
 #pragma unroll
     for (int u = 0; u < NM; ++u) load[u] = 0.0f;
+    // a job of another machine adds zero: a load is never -0, so that changes nothing, and only
+    // the addition itself is on the chain (branches took 56 cycles a job)
     int i = 0;
-#pragma unroll 2
-    for (; i + 4 <= n; i += 4) {
-        const int4 q = *reinterpret_cast<const int4*>(mid + i);
-        const float4 v = __ldg(reinterpret_cast<const float4*>(jt + i));
+#pragma unroll 1
+    for (; i + 16 <= n; i += 16) {
+        int4 q[4];
+        float4 v[4];
 #pragma unroll
-        for (int u = 0; u < NM; ++u) {
-            const int me = m0 + u * T;
-            if (q.x == me) load[u] = __fadd_rn(load[u], v.x);
-            if (q.y == me) load[u] = __fadd_rn(load[u], v.y);
-            if (q.z == me) load[u] = __fadd_rn(load[u], v.z);
-            if (q.w == me) load[u] = __fadd_rn(load[u], v.w);
+        for (int c = 0; c < 4; ++c) {
+            q[c] = *reinterpret_cast<const int4*>(mid + i + 4 * c);
+            v[c] = *reinterpret_cast<const float4*>(jt + i + 4 * c);
         }
+#pragma unroll
+        for (int c = 0; c < 4; ++c)
+#pragma unroll
+            for (int u = 0; u < NM; ++u) {
+                const int me = m0 + u * T;
+                load[u] = __fadd_rn(load[u], q[c].x == me ? v[c].x : 0.0f);
+                load[u] = __fadd_rn(load[u], q[c].y == me ? v[c].y : 0.0f);
+                load[u] = __fadd_rn(load[u], q[c].z == me ? v[c].z : 0.0f);
+                load[u] = __fadd_rn(load[u], q[c].w == me ? v[c].w : 0.0f);
+            }
     }
     for (; i < n; ++i)
 #pragma unroll
         for (int u = 0; u < NM; ++u)
-            if (mid[i] == m0 + u * T) load[u] = __fadd_rn(load[u], __ldg(jt + i));
+            if (mid[i] == m0 + u * T) load[u] = __fadd_rn(load[u], jt[i]);
     float best = -INFINITY;
 #pragma unroll
     for (int u = 0; u < NM; ++u)
@@ -709,7 +718,7 @@ __device__ __forceinline__ float jobsched_pass(const int32_t* mid, int n, const 
 }
 
 template <int T>
-__device__ __forceinline__ float jobsched_makespan(int n, const float* __restrict__ jt, int M, const RowBuf& s,
+__device__ __forceinline__ float jobsched_makespan(int n, const float* jt, int M, const RowBuf& s,
                                                    const RowGroup<T>& g) {
     float best = -INFINITY;
     for (int m0 = 0; m0 < M; m0 += 4 * T) {

@@ -25,12 +25,13 @@ namespace bk {
 constexpr size_t kSmSharedBytes = 228 * 1024;  // per SM; each CTA takes 1 KB more than it asks for
 constexpr size_t kRowSmemCap = 227 * 1024;  // opt-in dynamic shared memory per CTA
 
+// instance data that a CTA stages in shared memory: coordinates, or job times
 __host__ __device__ inline bool has_points(int kind) {
-    return kind == TSP_COORDS || kind == BITSP_COORDS || kind == MOVRP;
+    return kind == TSP_COORDS || kind == BITSP_COORDS || kind == MOVRP || kind == JOBSCHED;
 }
 
 static size_t points_bytes(int max_points, int kind) {
-    return row_align(max_points * 8u * (kind == BITSP_COORDS ? 2u : 1u));
+    return row_align(max_points * (kind == BITSP_COORDS ? 16u : kind == JOBSCHED ? 4u : 8u));
 }
 
 // Whether a row's keys stay in shared memory between the histogram and the scatter (14 bytes
@@ -134,7 +135,12 @@ __global__ void __launch_bounds__(T * max_groups(T), 1) row_kernel(RowLaunch L) 
             for (int i = threadIdx.x; i < (int)(sizeof(PopDesc) / 4); i += blockDim.x)
                 reinterpret_cast<uint32_t*>(&sd)[i] = from[i];
             __syncthreads();
-            if (L.stage_xy && has_points(sd.kind)) {
+            if (CLS == ROWS_KEYS) {
+                if (L.stage_xy && sd.kind == JOBSCHED) {
+                    for (int i = threadIdx.x; i < sd.n; i += blockDim.x) pts[i] = sd.jt[i];
+                    __syncthreads();
+                }
+            } else if (L.stage_xy && has_points(sd.kind)) {
                 const int npts = (sd.kind == TSP_COORDS) ? sd.n : sd.n + 1;
                 const float2* g0 = reinterpret_cast<const float2*>(sd.xy);
                 float2* d0 = reinterpret_cast<float2*>(pts);
@@ -450,7 +456,7 @@ __global__ void __launch_bounds__(T * max_groups(T), 1) row_kernel(RowLaunch L) 
                 zero_counters<T>(s, t);  // the terms lay over them
             } else {
                 g.sync();
-                res[0] = jobsched_makespan<T>(n, sd.jt, sd.machines, s, g);
+                res[0] = jobsched_makespan<T>(n, L.stage_xy ? pts : sd.jt, sd.machines, s, g);
             }
         } else if constexpr (TSPJ_ROWS) {
             sort_row<T, true>(n4, split, s, g, plain, keys_again);
@@ -567,9 +573,12 @@ int tile_candidates(int n, RowTile* out, int cap) {
     return c;
 }
 
-// the default: up to four groups a thread
-RowTile pick_tile(int n) {
+// the default: up to four groups a thread; one warp where a sum in index order takes most of
+// the time, which more threads do not share (job scheduling, n = 1000, P = 2048: 18 us a
+// generation's rows with 32 threads, 21 with 64, 36 with 128)
+RowTile pick_tile(int n, int kind) {
     if (n > row_max_n()) return RowTile{0, 0};
+    if ((kind == JOBSCHED || kind == CONTINUOUS) && tile_groups(32, n) <= 16) return RowTile{32, tile_groups(32, n)};
     for (int b = 32; b < 1024; b *= 2)
         if (tile_groups(b, n) <= 4) return RowTile{b, tile_groups(b, n)};
     return RowTile{1024, tile_groups(1024, n)};
