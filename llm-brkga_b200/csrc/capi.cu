@@ -248,14 +248,25 @@ static void tune_load_file() {
     std::fclose(f);
 }
 
-int32_t tune_lookup(int kind, int n, int rows, RowTile* t) {
+bool forced_tile(int n, RowTile* t) {
     if (const char* forced = std::getenv("BRKGA_TILE")) {
         int b = 0, g = 0;
         if (std::sscanf(forced, "%d,%d", &b, &g) == 2 && 4 * b * g >= n) {
             *t = RowTile{b, g};
-            return BRKGA_OK;
+            return true;
         }
     }
+    return false;
+}
+
+int32_t default_tile(int kind, int n, int pts, int rows, TunedTile* out) {
+    RowTile t{};
+    if (!forced_tile(n, &t)) t = pick_tile(n, kind);
+    return tile_setup(t, kind, n, pts, rows, out);
+}
+
+int32_t tune_lookup(int kind, int n, int rows, RowTile* t) {
+    if (forced_tile(n, t)) return BRKGA_OK;
     std::lock_guard<std::mutex> lk(g_tune_mu);
     tune_load_file();
     auto it = g_tune.find({cur_device(), kind, n, rows});

@@ -97,6 +97,8 @@ using namespace bk;
 
 // the longest captured run of plain generations is 2^kMaxRunLog
 constexpr int kMaxRunLog = 4;
+// generations of one evolve launch at most
+constexpr int kEvolveRun = 128;
 
 struct brkga_engine {
     std::mutex mu;
@@ -136,6 +138,9 @@ struct brkga_engine {
     size_t gstride = 0;
     int ls_count = 0;          // TSPJ local search: top ranks searched per island (0 = off)
     Task* d_tasks_ls = nullptr;
+    EvolvePlan evo;            // whole generations in one launch (groups 0: graphs of row and rank launches)
+    unsigned long long* evo_words = nullptr;
+    uint32_t evo_step = 0;
 };
 
 static RowLaunch base_launch(brkga_engine* e, int mode) {
@@ -228,6 +233,8 @@ static int32_t sync_descs_to_host(brkga_engine* e) {
     if (err != cudaSuccess) return cuda_fail(err, "engine stream");
     err = cudaMemcpy(e->hd.data(), e->dd, sizeof(PopDesc) * e->hd.size(), cudaMemcpyDeviceToHost);
     if (err != cudaSuccess) return cuda_fail(err, "descriptor read-back");
+    for (const PopDesc& d : e->hd)
+        if (d.stuck) return fail(BRKGA_ERR_TIMEOUT, "a wait between the launch's CTAs ran out; the population is not valid");
     return BRKGA_OK;
 }
 
@@ -335,6 +342,22 @@ int32_t brkga_create(brkga_problem* pbh, const brkga_params* params, brkga_engin
         d.cur = 0;
         d.gen = 0;
     }
+    // one population: whole generations per launch, where that is the faster way.  The parents of
+    // a generation are then drawn by the CTAs that use them
+    {
+        RowTile forced{};
+        const int threads = forced_tile(sh.n, &forced) ? forced.block : 0;
+        if (!sh.mo && sh.k == 1 && !row_needs_global(sh.n, points_of(*pd), pd->kind) &&
+            evolve_plan(pd->kind, sh.n, sh.Pi, threads, &e->evo)) {
+            if ((st = dalloc(e->pop, &p, (size_t)24 * sh.Pi)) != BRKGA_OK) {
+                destroy_engine(e);
+                return st;
+            }
+            e->evo_words = (unsigned long long*)p;
+            cudaMemsetAsync(p, 0, (size_t)24 * sh.Pi, e->stream);
+            e->hd[0].parents = nullptr;
+        }
+    }
     // TSPJ random 2-opt local search (the reference runs it in its island loop on
     // problems whose config has one: TSPJConfig, configs/tspj_config.hpp:69-136)
     if (!sh.mo && pd->kind == BRKGA_TSPJ && params->local_search_interval > 0 &&
@@ -421,8 +444,10 @@ int32_t brkga_create(brkga_problem* pbh, const brkga_params* params, brkga_engin
                 return st;
             }
         } else {
+            // engines that evolve in one launch use the tile for their first population only
             TunedTile tt;
-            st = autotune_tile(pd->kind, sh.n, pts, rows, e->stream, launch, &tt);
+            if (e->evo.groups > 0) st = default_tile(pd->kind, sh.n, pts, rows, &tt);
+            else st = autotune_tile(pd->kind, sh.n, pts, rows, e->stream, launch, &tt);
             if (st != BRKGA_OK) {
                 destroy_engine(e);
                 return st;
@@ -473,6 +498,7 @@ int32_t brkga_initialize(brkga_engine* e) {
     for (auto& d : e->hd) {
         d.cur = 0;
         d.gen = 0;
+        d.stuck = 0;
     }
     cudaError_t err = cudaMemcpyAsync(e->dd, e->hd.data(), sizeof(PopDesc) * e->hd.size(),
                                       cudaMemcpyHostToDevice, e->stream);
@@ -508,6 +534,22 @@ int32_t brkga_evolve(brkga_engine* e, int32_t generations) {
     cudaError_t err = cudaSuccess;
     int left = generations;
     NvtxRange all("brkga_evolve", e->gen + 1u, e->gen + (unsigned)generations);
+    while (e->evo.groups > 0 && left > 0 && err == cudaSuccess) {
+        // bounded launches: other streams' work gets its turn between them
+        const int step = std::min(left, kEvolveRun);
+        NvtxRange run("generations", e->gen + 1u, e->gen + (unsigned)step);
+        err = launch_evolve(e->evo, e->pop.pd->kind, e->pop.sh.n, points_of(*e->pop.pd), e->dd, step, e->evo_step,
+                            e->ls_count, e->pop.prm.local_search_moves, e->evo_words, e->pop.sh.Pi, e->stream);
+        if (err == cudaSuccess) e->evo_step += kEvolveSteps * (uint32_t)step;
+        if (err == cudaErrorCooperativeLaunchTooLarge) {
+            // fewer SMs than the device reports (a partitioned GPU): the launches below do
+            e->evo.groups = 0;
+            err = cudaSuccess;
+            break;
+        }
+        left -= step;
+        e->gen += (uint32_t)step;
+    }
     while (left > 0 && err == cudaSuccess) {
         // plain generations until (and excluding) the next special one, in captured runs of
         // 16, then 8, 4, 2, 1

@@ -97,6 +97,8 @@ struct TunedTile {
 };
 template <typename F>
 int32_t autotune_tile(int kind, int n, int pts, int rows, cudaStream_t stream, F&& launch, TunedTile* out);
+bool forced_tile(int n, RowTile* t);  // BRKGA_TILE, when it covers n
+int32_t default_tile(int kind, int n, int pts, int rows, TunedTile* out);
 int32_t tune_lookup(int kind, int n, int rows, RowTile* t);
 void tune_store(int kind, int n, int rows, const RowTile& t);
 int32_t tile_setup(const RowTile& t, int kind, int n, int pts, int rows, TunedTile* out);

@@ -92,6 +92,33 @@ cudaError_t launch_rows(const RowLaunch& L, int kind, const RowTile& tile, int g
 cudaError_t launch_rows_global(const RowLaunch& L, int kind, int grid, cudaStream_t s);
 // convenience for one-off launches: prepare + launch with an occupancy-sized grid
 cudaError_t launch_rows_auto(const RowLaunch& L, int kind, const RowTile& tile, cudaStream_t s);
+// bytes of instance data a CTA stages; whether rows keep their keys in shared memory; groups of
+// four keys a thread of a tile takes
+size_t points_bytes(int max_points, int kind);
+bool keep_keys(int kind);
+int tile_groups(int block, int n);
+
+// ---------------------------------------------------------------------------------------
+// whole generations of one single-objective population in one launch (evolve.cu)
+// ---------------------------------------------------------------------------------------
+struct EvolvePlan {
+    RowTile tile{};
+    int groups = 0;    // row groups per CTA (0: the population is not run this way)
+    int ctas = 0;
+    bool stage = false, keep = false;
+    size_t smem = 0;
+};
+// whether populations of P rows of n keys of this kind run in evolve launches, and how
+// (threads: per row, 0 = chosen by size)
+bool evolve_plan(int kind, int n, int P, int threads, EvolvePlan* out);
+// `gens` generations of the population at desc (its rows ranked): rows, elite partition, and for
+// TSPJ the local search of ls_count rows where due.  words: 3 P 64-bit words of device memory,
+// zero before the first launch; step0: the steps earlier launches took (kEvolveSteps a
+// generation).
+constexpr uint32_t kEvolveSteps = 2;
+cudaError_t launch_evolve(const EvolvePlan& p, int kind, int n, int max_points, PopDesc* desc, int gens, uint32_t step0,
+                          int ls_count, int ls_moves, unsigned long long* words, int P, cudaStream_t s);
+
 // raise the shared-memory limit of the sort kernels for populations of up to maxP rows
 cudaError_t prepare_sort(int maxP);
 // raise (never lower) the dynamic shared-memory limit of a kernel on the current device

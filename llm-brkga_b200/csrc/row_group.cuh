@@ -152,7 +152,7 @@ __device__ __noinline__ void rank_loop(const int32_t* sk, const uint16_t* si, ui
 }
 
 // equal keys in a thread's window: the window took them in position order; by index instead
-__device__ __noinline__ int tie_fix(const int32_t* sk, const uint16_t* si, int p) {
+static __device__ __noinline__ int tie_fix(const int32_t* sk, const uint16_t* si, int p) {
     const int32_t a = sk[p];
     const uint16_t x = si[p];
     int r = 0;
