@@ -137,11 +137,10 @@ struct PopDesc {
     int32_t* nrank;           // [2P] pool ranks; [0,P) the survivors'
     float* ncd;               // [2P] crowding distances
     int32_t* nsel;            // [P] survivor pool indices / unique list of the diversity pass
-    uint32_t* domS;           // [2P][domW] dominance rows
-    int32_t* domcnt;          // [2P] domination counts
+    uint32_t* domS;           // [2P][domW] dominance rows: bit j of row i set when j dominates i
+    int32_t* domcnt;          // [2P] ranks of the last peel
     int32_t* nu;              // diversity pass: unique count, P when nothing was rebuilt
-    int32_t* nord;            // [2][2P] pool points in (rank, objective o, index) order, then
-                              // [2P] the pool's dominator counts (zero between generations)
+    int32_t* nord;            // [2][2P] pool points in (rank, objective o, index) order
     int32_t* nft;             // front table of the last peel: [0] ranks, [1] cut rank (-1: none),
                               // [2 + r] first position of rank r in rank order, [2 + ranks] = N
     float* ncdp;              // [2P] crowding distance of every pool point

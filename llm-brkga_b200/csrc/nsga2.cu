@@ -136,32 +136,16 @@ struct DomArgs {
     const float* obj;     // raw mode
     int rawN, m;
     uint32_t* S;          // raw mode: [N][Wmax]
-    int32_t* cnt;         // raw mode: [N]
+    int32_t* cnt;         // raw mode: [N] dominator counts (null: not wanted)
     int Wmax;
+    int dominators;       // rows hold the points that dominate i (the row peel), not those i dominates
 };
 
 __global__ void dom_build_kernel(DomArgs a) {
-    const float* obj;
-    int N, m, Wmax;
-    uint32_t* S;
-    int32_t* cnt;
-    if (a.dd) {
-        const PopDesc& d = a.dd[blockIdx.y];
-        if (a.only_rebuilt && (!d.advanced || __ldg(d.nu) >= d.P)) return;
-        N = d.P;
-        m = d.m;
-        obj = d.fit[d.cur];
-        S = d.domS;
-        cnt = d.domcnt;
-        Wmax = d.domW;
-    } else {
-        N = a.rawN;
-        m = a.m;
-        obj = a.obj;
-        S = a.S;
-        cnt = a.cnt;
-        Wmax = a.Wmax;
-    }
+    const float* obj = a.obj;
+    const int N = a.rawN, m = a.m, Wmax = a.Wmax;
+    uint32_t* S = a.S;
+    int32_t* cnt = a.cnt;
     const int W = (N + 31) / 32;
     const int lane = threadIdx.x & 31;
     const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
@@ -181,10 +165,10 @@ __global__ void dom_build_kernel(DomArgs a) {
             }
             const uint32_t si = __ballot_sync(0xffffffffu, dij);
             const uint32_t di = __ballot_sync(0xffffffffu, dji);
-            if (lane == 0) S[(size_t)i * Wmax + w] = si;
+            if (lane == 0) S[(size_t)i * Wmax + w] = a.dominators ? di : si;
             c += __popc(di);
         }
-        if (lane == 0) cnt[i] = c;
+        if (lane == 0 && cnt) cnt[i] = c;
     }
 }
 
@@ -209,11 +193,6 @@ __device__ __forceinline__ void staged(int count, Ld ld, St st) {
     }
 }
 
-// A generation's pool (two objectives): the dominator counts are accumulated into a slot
-// after the two orders (nord + 2N, N = 2P), which is zero between generations: the peel
-// reads each count and clears it.
-__host__ __device__ inline int32_t* pool_counts(const PopDesc& d) { return d.nord + 4 * (size_t)d.P; }
-
 // 32 x 32 bit transpose across a warp: lane l holds row l on entry (bit c = element (l, c))
 // and column l on exit (bit r = element (r, l)); five exchange steps of halving blocks.
 __device__ __forceinline__ uint32_t warp_transpose32(uint32_t w, int lane) {
@@ -228,12 +207,11 @@ __device__ __forceinline__ uint32_t warp_transpose32(uint32_t w, int lane) {
     return w;
 }
 
-// The pool's dominance rows, each unordered pair of 32-point blocks (I <= J) visited once
-// by one warp: for row r of block I against lane j of block J the four compares give
-// both directions.  Row words: block I's rows at word J directly; block J's rows at word
-// I from the other direction's ballots by a bit transpose.  Dominator counts by atomic
-// adds into pool_counts (a diagonal block adds only once).  The same compares as
-// dom2_build_kernel, so the same matrix and counts bit for bit; half the pair tests.
+// The pool's dominator rows (row i, bit j: j dominates i), each unordered pair of 32-point
+// blocks (I <= J) visited once by one warp: for row r of block I against lane j of block J
+// the four compares give both directions.  Block I's rows at word J come from one
+// direction's ballots directly; block J's rows at word I from the other's by a bit
+// transpose.  The same compares as dom2_build_kernel, half the pair tests.
 constexpr int kSymWarps = 16;
 
 __global__ void __launch_bounds__(kSymWarps * 32) dom2_pool_kernel(PopDesc* dd) {
@@ -245,7 +223,6 @@ __global__ void __launch_bounds__(kSymWarps * 32) dom2_pool_kernel(PopDesc* dd) 
     const int T = W * (W + 1) / 2;
     const float2* __restrict__ o2 = reinterpret_cast<const float2*>(d.fit[d.cur]);
     uint32_t* const S = d.domS;
-    int32_t* const acc = pool_counts(d);
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     float2* const rows = srow[warp];
     // consecutive tiles go to different CTAs, so that every CTA (and SM) gets the same
@@ -280,32 +257,22 @@ __global__ void __launch_bounds__(kSymWarps * 32) dom2_pool_kernel(PopDesc* dd) 
         rows[lane] = oi;
         __syncwarp();
         uint32_t rw = 0u, cw = 0u;
-        int cj = 0;
 #pragma unroll 8
         for (int r = 0; r < 32; ++r) {
             const float2 a = rows[r];
             const bool gt0 = a.x > oj.x, gt1 = a.y > oj.y;
             const bool lt0 = a.x < oj.x, lt1 = a.y < oj.y;
-            const bool rdj = !gt0 && !gt1 && (lt0 || lt1);  // row 32 I + r dominates 32 J + lane
-            const uint32_t s1 = __ballot_sync(0xffffffffu, rdj);
-            const uint32_t s2 = __ballot_sync(0xffffffffu, !lt0 && !lt1 && (gt0 || gt1));
-            cj += rdj ? 1 : 0;
+            const uint32_t s1 = __ballot_sync(0xffffffffu, !gt0 && !gt1 && (lt0 || lt1));  // row r dominates lane
+            const uint32_t s2 = __ballot_sync(0xffffffffu, !lt0 && !lt1 && (gt0 || gt1));  // lane dominates row r
             if (lane == r) {
                 rw = s1;
                 cw = s2;
             }
         }
-        if (i < N) {
-            S[(size_t)i * Wmax + J] = rw;
-            const int c = __popc(cw);  // points of block J dominating i
-            if (c) atomicAdd(acc + i, c);
-        }
+        if (i < N) S[(size_t)i * Wmax + J] = cw;
         if (I != J) {
-            const uint32_t tw = warp_transpose32(cw, lane);  // row j, word I
-            if (j < N) {
-                S[(size_t)j * Wmax + I] = tw;
-                if (cj) atomicAdd(acc + j, cj);
-            }
+            const uint32_t tw = warp_transpose32(rw, lane);  // row j, word I
+            if (j < N) S[(size_t)j * Wmax + I] = tw;
         }
         I = nI;
         J = nJ;
@@ -333,7 +300,7 @@ __global__ void __launch_bounds__(kDom2Warps * 32) dom2_build_kernel(DomArgs a) 
         N = d.P;
         obj = d.fit[d.cur];
         S = d.domS;
-        cnt = d.domcnt;
+        cnt = nullptr;
         Wmax = d.domW;
     } else {
         N = a.rawN;
@@ -376,7 +343,7 @@ __global__ void __launch_bounds__(kDom2Warps * 32) dom2_build_kernel(DomArgs a) 
                 const uint32_t si = __ballot_sync(0xffffffffu, !gt0 && !gt1 && (lt0 || lt1));
                 const uint32_t di = __ballot_sync(0xffffffffu, !lt0 && !lt1 && (gt0 || gt1));
                 c[r] += __popc(di);
-                if (lane == (w & 31)) buf[r] = si;
+                if (lane == (w & 31)) buf[r] = a.dominators ? di : si;
             }
         }
         // lane l holds word 32 b + l of each row: one coalesced store per row
@@ -391,7 +358,7 @@ __global__ void __launch_bounds__(kDom2Warps * 32) dom2_build_kernel(DomArgs a) 
         for (int r = 0; r < kDom2Rows; ++r) cpart[cg][rg * kDom2Rows + r] = c[r];
     }
     __syncthreads();
-    if (threadIdx.x < RPC && row0 + (int)threadIdx.x < N) {
+    if (cnt && threadIdx.x < RPC && row0 + (int)threadIdx.x < N) {
         int sum = 0;
 #pragma unroll
         for (int g = 0; g < kDom2ColGroups; ++g) sum += cpart[g][threadIdx.x];
@@ -770,107 +737,148 @@ __device__ __forceinline__ bool select_active(const PopDesc& d, int mode) {
     return true;
 }
 
-// Ranks by bit-sliced peeling on a cluster of kPeelCluster CTAs per population.  CTA c
-// owns columns [512c, 512c + 512) (16 words): their count planes, and for every front the
-// sum of the member rows' words over those columns.  The front masks are exchanged through
-// distributed shared memory with one cluster barrier per front, so the dominance rows are
-// read by eight SMs instead of one.  Ranks -> domcnt[0, N).
+// Ranks by peeling, on one thread-block cluster per population.  A point's dominator row
+// stays in registers for the whole peel: eight lanes hold it, 4 WL bytes each, and a warp
+// 16 points.  A front is a bit mask of the points in it; a point's count of dominators left
+// drops by the population count of (its row and the front), doubled for the first front
+// (its points are listed twice); points at or below zero form the next front.  Each warp
+// sends its 16 bits of the next front into every CTA's shared memory, and one cluster
+// barrier a front completes the mask.  Nothing is merged across warps: summing the rows of a
+// front's members column by column instead (bit-sliced partial sums of eight warps, added in
+// sequence, then subtracted) took about 6 us a front at N = 4096.  Population counts issue
+// at a quarter of the rate of logic, so a lane's words are first added carry-save (16 words:
+// 5 counts).
 //
 // The pool of a generation (mode 0) is peeled only up to the front where the survivors
 // (rank-0 points counted twice) first exceed P: that front is cut by crowding, and no
 // later front is selected.  The points left then get that front's rank + 1 as one last
 // front.  Selection, crowding of every selected point and the ranks kept for the next
-// generation are the same as with every front peeled.
-constexpr int kPeelCluster = 8, kPeelWords = 16, kPeelThreads = 256;
-constexpr int kPeelSlices = kPeelThreads / kPeelWords, kPeelWarps = kPeelThreads / 32;
+// generation are the same as with every front peeled.  Ranks -> domcnt[0, N).
+constexpr int kPeelThreads = 512, kPeelWarpPoints = 16, kPeelPoints = kPeelThreads / 32 * kPeelWarpPoints;
 
-__global__ void __cluster_dims__(kPeelCluster, 1, 1) __launch_bounds__(kPeelThreads)
-    nsga_peel_cluster_kernel(PopDesc* dd, int mode) {
+// set bits of x[0, n) (n = 4, 8 or 16): carry-save adders, then a count per weight
+template <int n>
+__device__ __forceinline__ int count_bits(const uint32_t (&x)[n]) {
+    uint32_t one = 0u, two = 0u, four = 0u, eight = 0u;
+    int high = 0;
+    auto add3 = [](uint32_t& s, uint32_t b, uint32_t c) {  // s <- the sum bit; returns the carry
+        const uint32_t cy = (s & b) | (c & (s | b));
+        s = s ^ b ^ c;
+        return cy;
+    };
+#pragma unroll
+    for (int i = 0; i < n; i += 4) {
+        const uint32_t t0 = add3(one, x[i], x[i + 1]), t1 = add3(one, x[i + 2], x[i + 3]);
+        const uint32_t f = add3(two, t0, t1);
+        const uint32_t e = four & f;
+        four ^= f;
+        const uint32_t s16 = eight & e;
+        eight ^= e;
+        if (i == 12) high = 16 * __popc(s16);
+    }
+    int c = __popc(one) + 2 * __popc(two) + 4 * __popc(four);
+    if (n > 4) c += 8 * __popc(eight);
+    return c + high;
+}
+
+template <int WL>
+__global__ void __launch_bounds__(kPeelThreads, 1) nsga_peel_rows_kernel(PopDesc* dd, int mode) {
     dep_wait();
     namespace cg = cooperative_groups;
-    __shared__ uint32_t C[kCB][kPeelWords];  // count planes of the own words (two's complement)
-    __shared__ uint32_t A[kPeelWords], V[kPeelWords];
-    __shared__ uint32_t Floc[2][kPeelWords];  // own words of the next front, by front parity
-    __shared__ uint16_t list[kMaxPool];
-    __shared__ uint32_t s_nf[2];              // member count of front k, by front parity
-    __shared__ uint32_t part[kPeelWarps][kDB][kPeelWords];
-    __shared__ uint16_t r16[kPeelWords * 32];
+    constexpr int NW = 8 * WL;  // words of a front mask
+    __shared__ __align__(16) uint32_t F[2][NW];  // front k in F[k & 1]
     cg::cluster_group cluster = cg::this_cluster();
-    const int crank = (int)cluster.block_rank();
-    PopDesc& d = dd[blockIdx.x / kPeelCluster];
+    const int csize = (int)cluster.num_blocks(), crank = (int)cluster.block_rank();
+    PopDesc& d = dd[blockIdx.x / csize];
     if (!select_active(d, mode)) return;  // the same decision in every CTA of the cluster
     const int N = (mode == 0) ? 2 * d.P : d.P;
-    const int W = (N + 31) / 32;
-    const uint32_t* __restrict__ S = d.domS;
-    const int Wmax = d.domW;
-    const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
-    const int w0 = crank * kPeelWords;
-    // domination counts of the own columns -> count planes; a generation's pool takes them
-    // from the pool build's accumulator and leaves it zero for the next generation
-    int32_t* const pacc = (mode == 0) ? pool_counts(d) : nullptr;
-    for (int wl = warp; wl < kPeelWords; wl += kPeelWarps) {
-        const int w = w0 + wl, i = 32 * w + lane;
-        int c = 0;
-        if (w < W && i < N) {
-            if (pacc) {
-                c = pacc[i];
-                pacc[i] = 0;
-            } else {
-                c = __ldg(d.domcnt + i);
-            }
+    const int W = (N + 31) / 32, Wmax = d.domW;
+    const int t = threadIdx.x, lane = t & 31, warp = t >> 5, sub = lane & 7;
+    const int p0 = crank * kPeelPoints + warp * kPeelWarpPoints;  // the warp's points; step s: p0 + 4 s + lane / 8
+
+    uint32_t x[4][WL];
+#pragma unroll
+    for (int st = 0; st < 4; ++st) {
+        const int p = p0 + 4 * st + (lane >> 3);
+#pragma unroll
+        for (int c = 0; c < WL / 4; ++c) {
+            const int w = 32 * c + 4 * sub;
+            const uint4 v = (p < N && w < Wmax) ? __ldg(reinterpret_cast<const uint4*>(d.domS + (size_t)p * Wmax + w))
+                                                : make_uint4(0u, 0u, 0u, 0u);
+            x[st][4 * c] = v.x, x[st][4 * c + 1] = v.y, x[st][4 * c + 2] = v.z, x[st][4 * c + 3] = v.w;
+        }
+    }
+    // counts of the points' dominators in the mask F[b], two per packed pair: steps 0 | 1, 2 | 3
+    auto dominators_in = [&](int b, int (&cnt)[4]) {
+        uint32_t m[WL];
+#pragma unroll
+        for (int c = 0; c < WL / 4; ++c) {
+            const uint4 v = *reinterpret_cast<const uint4*>(&F[b][32 * c + 4 * sub]);
+            m[4 * c] = v.x, m[4 * c + 1] = v.y, m[4 * c + 2] = v.z, m[4 * c + 3] = v.w;
+        }
+        uint32_t pk[2];
+#pragma unroll
+        for (int st = 0; st < 4; ++st) {
+            uint32_t y[WL];
+#pragma unroll
+            for (int u = 0; u < WL; ++u) y[u] = x[st][u] & m[u];
+            const uint32_t c = (uint32_t)count_bits<WL>(y);
+            if (st & 1) pk[st >> 1] |= c << 16;
+            else pk[st >> 1] = c;
         }
 #pragma unroll
-        for (int b = 0; b < kCB; ++b) {
-            const uint32_t pl = __ballot_sync(0xffffffffu, (c >> b) & 1);
-            if (lane == 0) C[b][wl] = pl;
+        for (int o = 1; o < 8; o <<= 1) {
+            pk[0] += __shfl_xor_sync(0xffffffffu, pk[0], o);
+            pk[1] += __shfl_xor_sync(0xffffffffu, pk[1], o);
         }
-        const uint32_t v = __ballot_sync(0xffffffffu, w < W && i < N);
-        if (lane == 0) V[wl] = v;
-    }
-    __syncthreads();
-    // first front: zero counts
-    if (t < kPeelWords) {
-        uint32_t z = V[t];
+        cnt[0] = (int)(pk[0] & 0xFFFFu), cnt[1] = (int)(pk[0] >> 16);
+        cnt[2] = (int)(pk[1] & 0xFFFFu), cnt[3] = (int)(pk[1] >> 16);
+    };
+    // the warp's points at or below zero and not ranked yet, as 16 bits, into every CTA's mask
+    uint32_t ranked = 0u;  // bit 4 s + lane / 8
+    auto send_front = [&](int b, const int (&cnt)[4]) {
+        uint32_t bits = 0u;
 #pragma unroll
-        for (int b = 0; b < kCB; ++b) z &= ~C[b][t];
-        A[t] = z;
-        Floc[0][t] = z;
-        for (uint32_t x = z; x; x &= x - 1) r16[32 * t + __ffs(x) - 1] = 0;
-    }
-    if (t == 0) {
-        s_nf[0] = 0;
-        s_nf[1] = 0;
+        for (int st = 0; st < 4; ++st) {
+            const uint32_t v = __ballot_sync(0xffffffffu, cnt[st] <= 0 && p0 + 4 * st + (lane >> 3) < N);
+            bits |= ((v & 1u) | ((v >> 7) & 2u) | ((v >> 14) & 4u) | ((v >> 21) & 8u)) << (4 * st);
+        }
+        bits &= ~ranked;
+        if (lane < csize)
+            reinterpret_cast<uint16_t*>(cluster.map_shared_rank(&F[b][0], lane))[p0 / kPeelWarpPoints] = (uint16_t)bits;
+    };
+    // every point: the counts of all dominators.  (Words past N stay zero: rows may hold anything
+    // there, and no CTA writes them when the cluster covers fewer points than the mask.)
+    for (int w = t; w < NW; w += kPeelThreads) {
+        F[1][w] = (w < N / 32) ? 0xFFFFFFFFu : (w == N / 32 && (N & 31)) ? (1u << (N & 31)) - 1u : 0u;
+        F[0][w] = 0u;
     }
     cluster.sync();
-    constexpr int NW = kPeelCluster * kPeelWords;
-    int survivors = 0, rest = 0;
+    int left[4];
+    dominators_in(1, left);
+    send_front(0, left);
+    cluster.sync();
+    if (csize * kPeelPoints < 32 * NW)
+        for (int w = csize * (kPeelPoints / 32) + t; w < NW; w += kPeelThreads) F[1][w] = 0u;
+    __syncthreads();
+
+    int survivors = 0, rest = 0, start = 0;
     // thread 0 of the cluster's first CTA records the front table (start of each front in
     // rank order, the cut front) for the grid-wide crowding and placement of mode 0
     int32_t* const ft = (crank == 0 && t == 0) ? d.nft : nullptr;
-    int start = 0;
-    for (int k = 0; k < N; ++k) {
-        // the whole front k, gathered from every CTA of the cluster; its member list is
-        // filled through one shared-memory atomic per warp (the order of the list does
-        // not matter: the column sums, the crowding scan and the cut-front sort do not
-        // depend on it)
-        uint32_t fw = 0u;
-        if (t < NW) fw = cluster.map_shared_rank(&Floc[k & 1][0], t / kPeelWords)[t % kPeelWords];
-        {
-            const uint32_t pc = __popc(fw);
-            uint32_t inc = pc;  // inclusive prefix of the warp's counts
+    for (int k = 0;; ++k) {
+        const uint32_t* f = F[k & 1];
+        // the front's size, and the members before this warp's points
+        const int word = p0 / 32;
+        int total = 0, pre = 0;
 #pragma unroll
-            for (int o = 1; o < 32; o <<= 1) {
-                const uint32_t y = __shfl_up_sync(0xffffffffu, inc, o);
-                if (lane >= o) inc += y;
-            }
-            uint32_t wbase = 0u;
-            if (lane == 31 && inc) wbase = atomicAdd(&s_nf[k & 1], inc);
-            uint32_t base = __shfl_sync(0xffffffffu, wbase, 31) + inc - pc;
-            for (uint32_t x = fw; x; x &= x - 1) list[base++] = (uint16_t)(32 * t + __ffs(x) - 1);
-            if (t == 0) s_nf[(k + 1) & 1] = 0u;  // read by every thread before the last barrier
+        for (int c = 0; c < (NW + 31) / 32; ++c) {
+            const int w = 32 * c + lane;
+            const int pc = (w < W) ? __popc(f[w]) : 0;
+            total += pc;
+            pre += (w < word) ? pc : 0;
         }
-        __syncthreads();
-        const uint32_t nf = s_nf[k & 1];
+        const int nf = __reduce_add_sync(0xffffffffu, total);
         if (nf == 0) {  // every CTA sees the same front
             if (ft) {
                 ft[0] = k;
@@ -880,11 +888,18 @@ __global__ void __cluster_dims__(kPeelCluster, 1, 1) __launch_bounds__(kPeelThre
             break;
         }
         if (ft) ft[2 + k] = start;
-        if (crank == 0 && d.nlist)
-            for (int j = t; j < (int)nf; j += kPeelThreads) d.nlist[start + j] = list[j];
-        start += (int)nf;
+        const uint32_t mine = reinterpret_cast<const uint16_t*>(f)[p0 / kPeelWarpPoints];
+        if (mine) {  // the warp's members: their ranks, and their places in the list of fronts
+            pre = __reduce_add_sync(0xffffffffu, pre) + ((p0 & 16) ? __popc(f[word] & 0xFFFFu) : 0);
+            if (lane < 16 && ((mine >> lane) & 1u)) {
+                d.domcnt[p0 + lane] = k;
+                if (d.nlist) d.nlist[start + pre + __popc(mine & ((1u << lane) - 1u))] = p0 + lane;
+            }
+            ranked |= mine;
+        }
+        start += nf;
         if (mode == 0) {
-            survivors += (k == 0) ? 2 * (int)nf : (int)nf;
+            survivors += (k == 0) ? 2 * nf : nf;
             if (survivors > d.P) {
                 rest = k + 1;
                 if (ft) {  // the cut front k, then the points left as one last front
@@ -896,113 +911,47 @@ __global__ void __cluster_dims__(kPeelCluster, 1, 1) __launch_bounds__(kPeelThre
                 break;
             }
         }
-        // column sums over the front's rows: thread (word t % 16, slice t / 16); the member
-        // rows' words are loaded sixteen at a time (one L2 round trip for fronts of up to
-        // 256 members) into 5-plane counters
-        const int wl = t % kPeelWords, sl = t / kPeelWords, w = w0 + wl;
-        uint32_t acc[kDB];
+        int dec[4];
+        dominators_in(k & 1, dec);
 #pragma unroll
-        for (int b = 0; b < kDB; ++b) acc[b] = 0u;
-        if (w < W) {
-            constexpr int kBatch = 16, kSP = 5;  // a batch counts up to 16: 5 planes
-            for (int j0 = sl; j0 < (int)nf; j0 += kBatch * kPeelSlices) {
-                uint32_t xs[kBatch];
-#pragma unroll
-                for (int u = 0; u < kBatch; ++u) {
-                    const int j = j0 + u * kPeelSlices;
-                    xs[u] = (j < (int)nf) ? __ldg(S + (size_t)list[j] * Wmax + w) : 0u;
-                }
-                uint32_t sv[kSP];
-#pragma unroll
-                for (int b = 0; b < kSP; ++b) sv[b] = 0u;
-#pragma unroll
-                for (int u = 0; u < kBatch; ++u) {
-                    uint32_t c = xs[u];
-#pragma unroll
-                    for (int b = 0; b < kSP; ++b) {
-                        const uint32_t nc = sv[b] & c;
-                        sv[b] ^= c;
-                        c = nc;
-                    }
-                }
-                uint32_t cy = 0u;
-#pragma unroll
-                for (int b = 0; b < kSP; ++b) {
-                    const uint32_t x = acc[b], y = sv[b];
-                    acc[b] = x ^ y ^ cy;
-                    cy = (x & y) | (cy & (x ^ y));
-                }
-#pragma unroll
-                for (int b = kSP; b < kDB; ++b) {
-                    const uint32_t x = acc[b];
-                    acc[b] = x ^ cy;
-                    cy = x & cy;
-                }
-            }
-        }
-        {  // the two slices of a warp (lanes l and l ^ 16 share a word)
-            uint32_t cy = 0u;
-#pragma unroll
-            for (int b = 0; b < kDB; ++b) {
-                const uint32_t o = __shfl_xor_sync(0xffffffffu, acc[b], 16);
-                const uint32_t s2 = acc[b] ^ o ^ cy;
-                cy = (acc[b] & o) | (cy & (acc[b] ^ o));
-                acc[b] = s2;
-            }
-        }
-        if (lane < kPeelWords)
-#pragma unroll
-            for (int b = 0; b < kDB; ++b) part[warp][b][wl] = acc[b];
-        __syncthreads();
-        if (t < kPeelWords) {
-            uint32_t nz = 0u;
-            if (w0 + t < W) {
-                uint32_t sum[kDB];
-#pragma unroll
-                for (int b = 0; b < kDB; ++b) sum[b] = part[0][b][t];
-                for (int wp = 1; wp < kPeelWarps; ++wp) {
-                    uint32_t cy = 0u;
-#pragma unroll
-                    for (int b = 0; b < kDB; ++b) {
-                        const uint32_t x = sum[b], y = part[wp][b][t];
-                        sum[b] = x ^ y ^ cy;
-                        cy = (x & y) | (cy & (x ^ y));
-                    }
-                }
-                // decrement: doubled for the first front (its points are listed twice)
-                uint32_t dec[kCB];
-#pragma unroll
-                for (int b = 0; b < kCB; ++b) dec[b] = 0u;
-                if (k == 0) {
-#pragma unroll
-                    for (int b = 1; b < kCB; ++b) dec[b] = (b - 1 < kDB) ? sum[b - 1] : 0u;
-                } else {
-#pragma unroll
-                    for (int b = 0; b < kDB; ++b) dec[b] = sum[b];
-                }
-                uint32_t bor = 0u, any = 0u;
-#pragma unroll
-                for (int b = 0; b < kCB; ++b) {
-                    const uint32_t x = C[b][t];
-                    const uint32_t dd2 = x ^ dec[b] ^ bor;
-                    bor = (~x & dec[b]) | (~(x ^ dec[b]) & bor);
-                    C[b][t] = dd2;
-                    any |= dd2;
-                }
-                const uint32_t sign = C[kCB - 1][t];
-                nz = (sign | ~any) & ~A[t] & V[t];
-                A[t] |= nz;
-                for (uint32_t x = nz; x; x &= x - 1) r16[32 * t + __ffs(x) - 1] = (uint16_t)(k + 1);
-            }
-            Floc[(k + 1) & 1][t] = nz;
-        }
+        for (int st = 0; st < 4; ++st) left[st] -= (k == 0) ? 2 * dec[st] : dec[st];
+        send_front((k + 1) & 1, left);
         cluster.sync();
     }
-    cluster.sync();  // no CTA leaves while another may still read its front words
-    for (int x = t; x < kPeelWords * 32; x += kPeelThreads) {
-        const int i = 32 * w0 + x;
-        if (i < N) d.domcnt[i] = ((A[x >> 5] >> (x & 31)) & 1u) ? r16[x] : (uint16_t)rest;
+    if (lane < 16 && p0 + lane < N && !((ranked >> lane) & 1u)) d.domcnt[p0 + lane] = rest;
+}
+
+using PeelFn = void (*)(PopDesc*, int);
+
+// one cluster per population: a CTA for every 256 of its (at most maxN) points
+static cudaError_t launch_peel(PopDesc* dd, int npops, int maxN, int mode, cudaStream_t s) {
+    int csize = 1;
+    while (csize * kPeelPoints < maxN) csize *= 2;
+    if (csize > 16) return cudaErrorInvalidValue;
+    const PeelFn fn = maxN <= 1024   ? nsga_peel_rows_kernel<4>
+                      : maxN <= 2048 ? nsga_peel_rows_kernel<8>
+                                     : nsga_peel_rows_kernel<16>;
+    if (csize > 8) {
+        const cudaError_t e =
+            cudaFuncSetAttribute(reinterpret_cast<const void*>(fn), cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+        if (e != cudaSuccess) return e;
     }
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(npops * csize);
+    cfg.blockDim = dim3(kPeelThreads);
+    cfg.stream = s;
+    cudaLaunchAttribute at[2];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    at[1].id = cudaLaunchAttributeClusterDimension;
+    at[1].val.clusterDim.x = csize;
+    at[1].val.clusterDim.y = 1;
+    at[1].val.clusterDim.z = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 2;
+    const cudaError_t e = cudaLaunchKernelEx(&cfg, fn, dd, mode);
+    if (e != cudaSuccess) cudaGetLastError();
+    return e;
 }
 
 // The pool ordered by (rank, objective o, index) for o = blockIdx.y, by exact counting:
@@ -1511,6 +1460,7 @@ static cudaError_t launch_dom(PopDesc* dd, int npops, int maxN, int only_rebuilt
     std::memset(&a, 0, sizeof(a));
     a.dd = dd;
     a.only_rebuilt = only_rebuilt;
+    a.dominators = 1;
     return launch_dom2(a, maxN, npops, st);
 }
 
@@ -1523,7 +1473,7 @@ cudaError_t nsga_enqueue_select(PopDesc* dd, int npops, int maxP, int mode, cuda
     else
         e = launch_dom(dd, npops, maxN, mode == 2 ? 1 : 0, st);
     if (e != cudaSuccess) return e;
-    e = launch_dep(nsga_peel_cluster_kernel, dim3(npops * kPeelCluster), dim3(kPeelThreads), 0, st, dd, mode);
+    e = launch_peel(dd, npops, maxN, mode, st);
     if (e != cudaSuccess) return e;
     if (mode == 0) {
         // a generation's pool: crowding and whole fronts from each point's own front, then
@@ -1552,7 +1502,7 @@ cudaError_t nsga_enqueue_diversity(PopDesc* dd, int npops, int maxP, cudaStream_
 int32_t nsga_alloc(PopDesc& d, int P, double mut_rate, int div_interval, int Mn, std::vector<void*>& allocs,
                    size_t* bytes, cudaStream_t stream) {
     const int N = 2 * P;
-    const int W = (N + 31) / 32;
+    const int W = round_up((N + 31) / 32, 4);  // dominance rows of whole 16-byte words
     auto get = [&](size_t b, void** p) -> int32_t {
         int32_t rc = dev_alloc(p, b ? b : 16, stream);
         if (rc != BRKGA_OK) return rc;
@@ -1574,12 +1524,8 @@ int32_t nsga_alloc(PopDesc& d, int P, double mut_rate, int div_interval, int Mn,
     d.domcnt = (int32_t*)p;
     if ((st = get(16, &p)) != BRKGA_OK) return st;
     d.nu = (int32_t*)p;
-    if ((st = get((size_t)3 * N * 4, &p)) != BRKGA_OK) return st;  // two orders, then the pool counts
+    if ((st = get((size_t)2 * N * 4, &p)) != BRKGA_OK) return st;
     d.nord = (int32_t*)p;
-    if (cudaMemsetAsync(d.nord + 2 * (size_t)N, 0, (size_t)N * 4, stream) != cudaSuccess) {
-        cudaGetLastError();
-        return fail(BRKGA_ERR_CUDA, "NSGA-II state initialisation");
-    }
     if ((st = get((size_t)(N + 4) * 4, &p)) != BRKGA_OK) return st;
     d.nft = (int32_t*)p;
     if ((st = get((size_t)N * 4, &p)) != BRKGA_OK) return st;
@@ -1873,7 +1819,8 @@ int32_t brkga_pareto_rank_bitmatrix(const float* d_obj, int32_t N, int32_t m, in
     if (N == 0) return BRKGA_OK;
     if (N > 8192) return fail(BRKGA_ERR_UNSUPPORTED, "more than 8192 points");
     cudaStream_t st = (cudaStream_t)stream;
-    const int W = (N + 31) / 32;
+    const bool rows = N <= kMaxPool;  // ranks by the engine's row peel; larger sets by one CTA's column peel
+    const int W = rows ? round_up((N + 31) / 32, 4) : (N + 31) / 32;
     const size_t sbytes = (size_t)N * W * 4, cbytes = (size_t)N * 4;
     const size_t doff = ((sbytes + cbytes + 255) / 256) * 256;  // a descriptor for the cluster peel
     std::lock_guard<std::mutex> lk(g_op_mu);
@@ -1888,6 +1835,8 @@ int32_t brkga_pareto_rank_bitmatrix(const float* d_obj, int32_t N, int32_t m, in
     a.S = (uint32_t*)buf;
     a.cnt = (int32_t*)((char*)buf + sbytes);
     a.Wmax = W;
+    a.dominators = rows ? 1 : 0;
+    if (rows) a.cnt = nullptr;
     cudaError_t e;
     if (m == 2) {
         e = launch_dom2(a, N, 1, st);
@@ -1896,23 +1845,19 @@ int32_t brkga_pareto_rank_bitmatrix(const float* d_obj, int32_t N, int32_t m, in
         e = cudaGetLastError();
     }
     if (e != cudaSuccess) return cuda_fail(e, "dominance launch");
-    if (N <= kMaxPool) {
-        // the engine's peel on a cluster of CTAs (ranks left in the counts), as for a
-        // population of N rows in mode 1
+    if (rows) {
+        // as for a population of N rows in mode 1, the ranks straight into the caller's buffer
         PopDesc hd;
         std::memset(&hd, 0, sizeof(hd));
         hd.P = N;
         hd.m = m;
         hd.domS = a.S;
         hd.domW = W;
-        hd.domcnt = a.cnt;
+        hd.domcnt = d_rank;
         PopDesc* dd = reinterpret_cast<PopDesc*>((char*)buf + doff);
         if ((e = cudaMemcpyAsync(dd, &hd, sizeof(hd), cudaMemcpyHostToDevice, st)) != cudaSuccess)
             return cuda_fail(e, "peel descriptor");
-        nsga_peel_cluster_kernel<<<kPeelCluster, kPeelThreads, 0, st>>>(dd, 1);
-        if ((e = cudaGetLastError()) != cudaSuccess) return cuda_fail(e, "peel launch");
-        if ((e = cudaMemcpyAsync(d_rank, a.cnt, cbytes, cudaMemcpyDeviceToDevice, st)) != cudaSuccess)
-            return cuda_fail(e, "rank copy");
+        if ((e = launch_peel(dd, 1, N, 1, st)) != cudaSuccess) return cuda_fail(e, "peel launch");
     } else {
         const size_t smem = (((size_t)N * 2 + 15) / 16) * 16 + peel_smem_bytes(N);
         if ((e = raise_smem_limit(reinterpret_cast<const void*>(peel_op_kernel), smem)) != cudaSuccess)
