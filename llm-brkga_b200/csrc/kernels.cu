@@ -1,19 +1,7 @@
-// kernels.cu -- the per-generation hot path on sm_100a.
-//
-// One CTA owns one chromosome row at a time (persistent grid, rows strided over CTAs):
-//   1. build the row in registers: elite copy, biased crossover of two parent rows
-//      (128-bit loads, Philox coins), mutant fill, or a load of given keys;
-//   2. write it to the next population buffer (128-bit stores);
-//   3. decode it: stable argsort of the keys in shared memory -- a bucket scatter
-//      (bucket = floor(key * B), monotone in key) followed by an exact rank inside each
-//      bucket by (key, index), so ties go to the lower index exactly like the
-//      reference's std::sort over (key, index) pairs (configs/tsp_config.hpp:206-225);
-//   4. fitness from the permutation: closed tour length from coordinates staged in
-//      shared memory (or a distance matrix), the depot tour of the bi-objective TSP,
-//      or the knapsack decoders; FP32 tour sums use one fixed order (256 virtual lanes,
-//      xor butterflies, fixed 8-way tree) that the oracle restates bit for bit.
-// The elite partition ranks (fitness key, row) composites by exact counting across the
-// grid (rank_kernel below).
+// kernels.cu -- rows beyond shared memory (row_kernel_big), the elite partition (rank_kernel)
+// and island migration.  The fused row kernel is in rows.cu, whole generations in one launch
+// in evolve.cu.  The elite partition ranks (fitness key, row) composites by exact counting
+// across the grid.
 #include <climits>
 #include <cstdio>
 #include <map>
@@ -21,25 +9,11 @@
 #include <utility>
 
 #include "kernels.h"
+#include "row_group.cuh"
 
 namespace bk {
 
 __host__ __device__ inline size_t align_up(size_t x, size_t a) { return (x + a - 1) / a * a; }
-
-__device__ __forceinline__ int bucket_of(float key, float nbf, int nb) {
-    // monotone in okey order: negatives -> 0; [0,1) -> floor(key * nb); >= 1, +inf, NaN -> nb-1
-    if (!(key >= 0.0f)) return (key != key) ? nb - 1 : 0;
-    const float t = __fmul_rn(key, nbf);
-    const int b = (t < nbf) ? (int)t : nb - 1;
-    return b < nb - 1 ? b : nb - 1;
-}
-
-// The exact rank inside a bucket scans the bucket, so its cost is the sum of the squared
-// bucket sizes.  Keys in [0,1) spread over about one per bucket; equal keys, keys outside
-// [0,1) (one bucket each side) or NaNs (the last bucket) pile into few buckets.  A row with
-// a bucket above kHeavyBucket keys is sorted instead by an ascending bitonic network over
-// its composites: O(n log^2 n) on any input, and the same (key, index) order.
-constexpr uint32_t kHeavyBucket = 32;
 
 // Ascending sort of a[0, n) (shared or global memory) by the whole block, any n: the
 // bitonic network in its one-direction form (each merge of size k first compares i with
@@ -96,62 +70,6 @@ __device__ __noinline__ void heavy_row_perm(unsigned long long* sc, int32_t* per
 // ---------------------------------------------------------------------------------------
 // fitness
 // ---------------------------------------------------------------------------------------
-// Euclidean edge exactly as the reference builds its matrix (configs/tsp_config.hpp:366-368):
-// float dx, dy; sqrt(dx*dx + dy*dy), no contraction, correctly rounded sqrt
-__device__ __forceinline__ float edge_xy(const float* xy, int a, int b) {
-    const float2 pa = reinterpret_cast<const float2*>(xy)[a];
-    const float2 pb = reinterpret_cast<const float2*>(xy)[b];
-    const float dx = __fsub_rn(pa.x, pb.x);
-    const float dy = __fsub_rn(pa.y, pb.y);
-    return __fsqrt_rn(__fadd_rn(__fmul_rn(dx, dx), __fmul_rn(dy, dy)));
-}
-
-// canonical FP32 sum of nedges edge terms: 256 virtual lanes, xor butterflies inside each
-// group of 32 lanes, fixed tree over the 8 group totals
-template <int BLOCK, int NOBJ, typename EdgeF>
-__device__ __forceinline__ void canon_sum(int nedges, EdgeF edge, float* red, float* out) {
-    constexpr int LPT = BLOCK >= 256 ? 1 : 256 / BLOCK;
-    const int t = threadIdx.x, lane = t & 31;
-    float acc[LPT][NOBJ];
-#pragma unroll
-    for (int j = 0; j < LPT; ++j) {
-#pragma unroll
-        for (int o = 0; o < NOBJ; ++o) acc[j][o] = 0.0f;
-        const int vl = t + j * BLOCK;
-        if (vl < 256) {
-            for (int e = vl; e < nedges; e += 256) {
-                float d[NOBJ];
-                edge(e, d);
-#pragma unroll
-                for (int o = 0; o < NOBJ; ++o) acc[j][o] = __fadd_rn(acc[j][o], d[o]);
-            }
-        }
-    }
-#pragma unroll
-    for (int m = 16; m >= 1; m >>= 1)
-#pragma unroll
-        for (int j = 0; j < LPT; ++j)
-#pragma unroll
-            for (int o = 0; o < NOBJ; ++o) acc[j][o] = __fadd_rn(acc[j][o], __shfl_xor_sync(0xffffffffu, acc[j][o], m));
-    if (lane == 0) {
-#pragma unroll
-        for (int j = 0; j < LPT; ++j) {
-            const int vl = t + j * BLOCK;
-            if (vl < 256) {
-#pragma unroll
-                for (int o = 0; o < NOBJ; ++o) red[o * 8 + (vl >> 5)] = acc[j][o];
-            }
-        }
-    }
-    __syncthreads();
-#pragma unroll
-    for (int o = 0; o < NOBJ; ++o) {
-        const float* g = red + o * 8;
-        out[o] = __fadd_rn(__fadd_rn(__fadd_rn(g[0], g[1]), __fadd_rn(g[2], g[3])),
-                           __fadd_rn(__fadd_rn(g[4], g[5]), __fadd_rn(g[6], g[7])));
-    }
-}
-
 // exclusive block scan of two 64-bit values at once (red: 64 entries)
 template <int BLOCK>
 __device__ __forceinline__ void block_excl_scan_ll2(long long a, long long b, long long* red, long long* ea,
@@ -409,37 +327,262 @@ __device__ __forceinline__ int tourn(int i1, int i2, const int32_t* rank, const 
 }
 
 // ---------------------------------------------------------------------------------------
-// rows beyond shared memory: the same build, bucket argsort and canonical sums, with the
-// sort's counters, composites and permutation in a per-CTA slice of global scratch
-// (L2-resident at these sizes) and the keys re-read from the row between passes.  One CTA
-// of 1024 threads per row; results equal the in-shared-memory kernel's bit for bit (the
-// sort order and the summation order do not depend on the tile).
+// rows beyond shared memory: the same build and canonical sums, one CTA per row.  The argsort
+// takes two levels: the row's keys are dealt to 4096 bins of the key range (a histogram and
+// cursors in shared memory; (key, gene) pairs to global scratch, L2-resident), and runs of
+// bins of up to kBigChunk keys are sorted in shared memory by the row kernel's argsort, one
+// after the other.  Equal keys go by gene, so results equal the other kernel's bit for bit.
+// Tours over coordinates are summed chunk by chunk: a point is fetched once, its edges are
+// formed from shared memory, and the 256 virtual lanes carry their sums from chunk to chunk.
+// With every counter, slot and composite of the row in global scratch instead, n = 65 536,
+// P = 512 took 3.2 ms (a dependent L2 round trip per key and step).  One CTA an SM: two of half
+// the size put 230 MB of scratch in flight, past L2, and took 1.3 ms.
 // ---------------------------------------------------------------------------------------
 constexpr int kBigBlock = 1024;
+constexpr int kBigBins = 4096;    // four a thread
+constexpr int kBigChunk = 10240;  // 18 bytes a key and a counter for each: 218 KB with the bins
+constexpr int kBigEdges = 8192;   // edge terms between two sums where the order comes from perm
 
-__host__ __device__ inline size_t big_cnt_bytes(int max_n) {
-    return align_up((size_t)(round_up(max_n, kBigBlock) + 1) * 4, 256);
-}
 __host__ __device__ inline size_t big_perm_bytes(int max_n) { return align_up((size_t)max_n * 4, 256); }
 
-size_t row_global_stride(int max_n) { return big_cnt_bytes(max_n) + big_perm_bytes(max_n) + align_up((size_t)max_n * 8, 256); }
+size_t row_global_stride(int max_n) { return big_perm_bytes(max_n) + align_up((size_t)max_n * 8, 256); }
 
-__global__ void __launch_bounds__(kBigBlock) row_kernel_big(RowLaunch L) {
+// the row slice (its kept keys widened to (key, gene) pairs), bins, first bin of each chunk
+__host__ __device__ inline uint32_t big_slice_bytes() { return row_slice_bytes(kBigBlock, kBigChunk, false); }
+static size_t big_smem_bytes() { return big_slice_bytes() + kBigChunk * 8 + kBigBins * 4 + kBigBins * 2; }
+
+// f(key, index) for every key of key[0, n) by a block of T threads: 128-bit loads, two of a thread
+// in flight ahead of the keys it works on, where the row is aligned
+template <int T, typename F>
+__device__ __forceinline__ void for_keys(const float* key, int n, int t, F f) {
+    int done = 0;
+    if ((reinterpret_cast<uintptr_t>(key) & 15) == 0) {
+        const float4* k4 = reinterpret_cast<const float4*>(key);
+        const int n4 = n / 4, rounds = n4 / T;
+        float4 a = make_float4(0.f, 0.f, 0.f, 0.f), b = a;
+        if (rounds > 0) a = k4[t];
+        if (rounds > 1) b = k4[t + T];
+        for (int r = 0; r < rounds; ++r) {
+            const float4 k = a;
+            const int i = 4 * (t + r * T);
+            a = b;
+            if (r + 2 < rounds) b = k4[t + (r + 2) * T];
+            f(k.x, i);
+            f(k.y, i + 1);
+            f(k.z, i + 2);
+            f(k.w, i + 3);
+        }
+        done = 4 * rounds * T;
+    }
+    for (int i = done + t; i < n; i += T) f(key[i], i);
+}
+
+// Stable argsort of key[0, n): done(p0, m) is called for each chunk in turn, by the whole block,
+// positions [p0, p0 + m) holding indices kin[s.perm[p - p0]].y (s.perm and kin are the chunk's;
+// the scratch behind s.perm is free).  False, before any call, when a bin holds more than half
+// a chunk, as equal or extreme keys do.
+template <typename DoneF>
+__device__ __forceinline__ bool long_argsort(const float* key, int n, uint2* sc, const RowBuf& s, uint2* kin,
+                                             uint32_t* bins, uint16_t* first_bin, const RowGroup<kBigBlock>& g,
+                                             DoneF done) {
+    constexpr int T = kBigBlock;
+    const int t = g.tid, lane = t & 31, warp = t >> 5;
+    uint4* b4 = reinterpret_cast<uint4*>(bins);
+    b4[t] = make_uint4(0u, 0u, 0u, 0u);
+    __syncthreads();
+    for_keys<T>(key, n, t, [&](float k, int) { atomicAdd(&bins[key_bucket(k, (float)kBigBins, kBigBins)], 1u); });
+    __syncthreads();
+    uint32_t* red = reinterpret_cast<uint32_t*>(s.red);
+    const uint4 c = b4[t];
+    const uint32_t sum = c.x + c.y + c.z + c.w;
+    uint32_t x = sum, big = __reduce_max_sync(0xffffffffu, max(max(c.x, c.y), max(c.z, c.w)));
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
+        if (lane >= o) x += y;
+    }
+    if (lane == 31) {
+        red[warp] = x;
+        red[32 + warp] = big;
+    }
+    __syncthreads();
+    const uint32_t v = (lane < T / 32) ? red[lane] : 0u;
+    const uint32_t start = x - sum + __reduce_add_sync(0xffffffffu, (lane < warp) ? v : 0u);
+    big = __reduce_max_sync(0xffffffffu, (lane < T / 32) ? red[32 + lane] : 0u);
+    if (big > kBigChunk / 2) {
+        __syncthreads();
+        return false;
+    }
+    const uint4 o = make_uint4(start, start + c.x, start + c.x + c.y, start + c.x + c.y + c.z);
+    b4[t] = o;
+    __syncthreads();
+    // chunk of a bin: its start over (kBigChunk - the largest bin), so a chunk's bins hold at
+    // most kBigChunk keys; starts grow by less than that, so every chunk has a first bin
+    const uint32_t span = kBigChunk - big;
+    {
+        const uint32_t st[4] = {o.x, o.y, o.z, o.w};
+        uint32_t before = t ? bins[4 * t - 1] / span : 0xFFFFFFFFu;
+#pragma unroll
+        for (int l = 0; l < 4; ++l) {
+            const uint32_t id = st[l] / span;
+            if (id != before) first_bin[id] = (uint16_t)(4 * t + l);
+            before = id;
+        }
+        if (t == T - 1) red[0] = before + 1u;
+    }
+    __syncthreads();
+    const int chunks = (int)red[0];
+    // Few chunks: each picks its keys out of the row, read again (L2, coalesced).  Many: the
+    // (key, gene) pairs are dealt to their bins in global scratch first, a 32-byte sector for
+    // each.  (n = 65 536, 7 chunks: dealing took 90 K cycles a row, 250 K with the scratch not in
+    // L2, and 50 K to read back; the seven passes take 154 K whatever is in L2.)
+    const bool deal = chunks > 12;
+    if (deal) {
+        for_keys<T>(key, n, t, [&](float k, int i) {
+            sc[atomicAdd(&bins[key_bucket(k, (float)kBigBins, kBigBins)], 1u)] =
+                make_uint2(__float_as_uint(k), (uint32_t)i);
+        });
+        __syncthreads();  // a bin's cursor now stands at the next bin's start
+    }
+    for (int ch = 0; ch < chunks; ++ch) {
+        const int b0 = first_bin[ch], b1 = (ch + 1 < chunks) ? first_bin[ch + 1] : kBigBins;
+        int p0, p1;
+        if (deal) {
+            p0 = b0 ? (int)bins[b0 - 1] : 0;
+            p1 = (int)bins[b1 - 1];
+        } else {
+            p0 = (int)bins[b0];  // not moved yet: only earlier chunks' cursors are
+            p1 = (b1 < kBigBins) ? (int)bins[b1] : n;
+        }
+        const int m = p1 - p0, m4 = round_up(m, 4);
+        if (m == 0) continue;
+        const float lo = (float)b0, scale = __fdiv_rn((float)s.nb, (float)(b1 - b0));
+        // monotone over the chunk's key range
+        auto bucket = [&](float k, int nb) {
+            const float f = __fmul_rn(__fsub_rn(__fmul_rn(k, (float)kBigBins), lo), scale);
+            return max((int)fminf(f, (float)nb - 1.0f), 0);
+        };
+        zero_counters<T>(s, t);
+        if (t == 0) red[64] = 0u;
+        __syncthreads();
+        if (deal) {
+            const uint2* part = sc + p0;
+            for (int p = t; p < m; p += T) kin[p] = part[p];
+        } else {
+            // bins are powers of two wide, so a chunk's keys are those between two exact bounds; NaN
+            // belongs to the last.  A thread counts its keys of the round, the warp adds up and takes
+            // its places with one atomic: a shared atomic takes the SM about eight cycles whatever
+            // its lanes, so one per key and pass (a bin's cursor) took 25 K cycles a pass
+            const float from = b0 ? (float)b0 / (float)kBigBins : -INFINITY;
+            const float to = (float)b1 / (float)kBigBins;
+            const bool last = b1 == kBigBins;
+            auto mine = [&](float k) { return !(k < from) && (last || k < to); };
+            constexpr int U = 8;  // keys a thread and round
+            float ahead[U];       // the next round's keys are on their way
+            const int rounds = (n + U * T - 1) / (U * T);
+            auto fetch = [&](int i0) {
+#pragma unroll
+                for (int u = 0; u < U; ++u) ahead[u] = (i0 + u * T < n) ? key[i0 + u * T] : 0.0f;
+            };
+            fetch(t);
+            for (int r = 0; r < rounds; ++r) {
+                const int i0 = t + r * U * T;
+                float k[U];
+                int c = 0;
+#pragma unroll
+                for (int u = 0; u < U; ++u) k[u] = ahead[u];
+                if (r + 1 < rounds) fetch(i0 + U * T);
+                const bool whole = (r + 1) * U * T <= n;
+#pragma unroll
+                for (int u = 0; u < U; ++u) c += (mine(k[u]) && (whole || i0 + u * T < n)) ? 1 : 0;
+                int x = c;
+#pragma unroll
+                for (int o = 1; o < 32; o <<= 1) {
+                    const int y = __shfl_up_sync(0xffffffffu, x, o);
+                    if (lane >= o) x += y;
+                }
+                uint32_t at = 0u;
+                if (lane == 31 && x) at = atomicAdd(&red[64], (uint32_t)x);
+                at = __shfl_sync(0xffffffffu, at, 31) + (uint32_t)(x - c);
+#pragma unroll
+                for (int u = 0; u < U; ++u)
+                    if (mine(k[u]) && (whole || i0 + u * T < n))
+                        kin[at++] = make_uint2(__float_as_uint(k[u]), (uint32_t)(i0 + u * T));
+            }
+        }
+        if (t < m4 - m) kin[m + t] = make_uint2(0x7FFFFFFFu, 0xFFFFFFFFu);
+        __syncthreads();
+        auto keys = [&](int q) {
+            const uint4 u = reinterpret_cast<const uint4*>(kin)[2 * q], v = reinterpret_cast<const uint4*>(kin)[2 * q + 1];
+            return make_float4(__uint_as_float(u.x), __uint_as_float(u.z), __uint_as_float(v.x), __uint_as_float(v.z));
+        };
+        for (int q = t; 4 * q < m; q += T) count_keys<false>(keys(q), q, m4, s, bucket);
+        sort_row<T, false>(m4, m4, s, g, bucket, keys, kin, m);
+        done(p0, m);
+        __syncthreads();
+    }
+    return true;
+}
+
+// the sums of the 256 virtual lanes (threads 0 .. 255) in the canonical order: butterflies in
+// groups of 32, a fixed tree over the groups
+__device__ float lane_tree(float acc, float* red, int t) {
+#pragma unroll
+    for (int o = 16; o >= 1; o >>= 1) acc = __fadd_rn(acc, __shfl_xor_sync(0xffffffffu, acc, o));
+    if (t < 256 && (t & 31) == 0) red[t >> 5] = acc;
+    __syncthreads();
+    const float v = __fadd_rn(__fadd_rn(__fadd_rn(red[0], red[1]), __fadd_rn(red[2], red[3])),
+                              __fadd_rn(__fadd_rn(red[4], red[5]), __fadd_rn(red[6], red[7])));
+    __syncthreads();
+    return v;
+}
+
+// canonical sum of a tour's edges in perm (global): every thread forms edge terms, kBigEdges at a
+// time in shared memory, then the 256 virtual lanes add theirs in order.  CLOSED as in tour_edges.
+template <bool CLOSED, typename EdgeF>
+__device__ float long_tour(int m, const int32_t* perm, EdgeF edge, float* ed, float* red, int t) {
+    constexpr int T = kBigBlock;
+    const int edges = CLOSED ? m : m + 1;
+    auto stop = [&](int j) {  // the j-th stop of the tour: edge e joins stops e and e + 1
+        if (CLOSED) return perm[j < m ? j : 0];
+        return (j == 0 || j > m) ? 0 : perm[j - 1] + 1;
+    };
+    float acc = 0.0f;
+    for (int e0 = 0; e0 < edges; e0 += kBigEdges) {
+        const int cnt = min(kBigEdges, edges - e0);
+        for (int c = t; 4 * c < cnt; c += T) {
+            int id[5];
+#pragma unroll
+            for (int i = 0; i < 5; ++i) id[i] = stop(min(e0 + 4 * c + i, edges));
+            float4 d;
+            edge(id, &d.x);
+            reinterpret_cast<float4*>(ed)[c] = d;
+        }
+        __syncthreads();
+        if (t < 256)
+            for (int e = t; e < cnt; e += 256) acc = __fadd_rn(acc, ed[e]);
+        __syncthreads();
+    }
+    return lane_tree(acc, red, t);
+}
+
+__global__ void __launch_bounds__(kBigBlock, 1) row_kernel_big(RowLaunch L) {
     constexpr int BLOCK = kBigBlock;
+    extern __shared__ __align__(16) unsigned char smem_raw[];
     __shared__ PopDesc sd;
-    __shared__ uint32_t warp_tot[32];
     __shared__ long long red_ll[64];
     __shared__ float red_f[32];
     __shared__ long long misc[4];
     const int t = threadIdx.x;
+    const RowGroup<BLOCK> g;
+    const RowBuf s = row_carve(smem_raw, BLOCK, kBigChunk, false);
+    uint2* kin = reinterpret_cast<uint2*>(smem_raw + big_slice_bytes());
+    uint32_t* bins = reinterpret_cast<uint32_t*>(kin + kBigChunk);
+    uint16_t* first_bin = reinterpret_cast<uint16_t*>(bins + kBigBins);
+    float* ed = reinterpret_cast<float*>(smem_raw);
     unsigned char* base = static_cast<unsigned char*>(L.gscratch) + (size_t)blockIdx.x * L.gstride;
-    uint32_t* cnt = reinterpret_cast<uint32_t*>(base);                               // [NB + 1]
-    int32_t* perm = reinterpret_cast<int32_t*>(base + big_cnt_bytes(L.max_n));       // slots, then the permutation
-    unsigned long long* sc =
-        reinterpret_cast<unsigned long long*>(base + big_cnt_bytes(L.max_n) + big_perm_bytes(L.max_n));
-    const int NBmax = round_up(L.max_n, BLOCK);
-    for (int j = t; j <= NBmax; j += BLOCK) cnt[j] = 0u;
-    __syncthreads();
+    int32_t* perm = reinterpret_cast<int32_t*>(base);
+    unsigned long long* sc = reinterpret_cast<unsigned long long*>(base + big_perm_bytes(L.max_n));
     int cur_pid = -1;
 
     for (int task = blockIdx.x; task < L.ntasks; task += gridDim.x) {
@@ -603,84 +746,121 @@ __global__ void __launch_bounds__(kBigBlock) row_kernel_big(RowLaunch L) {
         } else if (kind == JOBSCHED) {
             res[0] = jobsched_makespan<BLOCK>(row, n, sd.jt, sd.machines, red_f);
         } else {
-            // stable argsort by (okey, index): bucket histogram, scan, scatter, rank in bucket
-            const int NB = round_up(n, BLOCK);
-            const int split = (kind == TSPJ) ? n / 2 : n;  // two segments: buckets split in halves
-            const int nbs = (split < n) ? NB / 2 : NB;
-            const float nbf = (float)nbs;
-            auto bucket = [&](float k, int i) { return bucket_of(k, nbf, nbs) + ((i >= split) ? nbs : 0); };
-            for (int i = t; i < n; i += BLOCK) perm[i] = (int32_t)atomicAdd(&cnt[bucket(row[i], i)], 1u);
-            __syncthreads();
-            bool heavy;
-            {
-                const int ch = NB / BLOCK;
-                uint32_t sum = 0, big = 0;
-                for (int j = t * ch; j < t * ch + ch; ++j) {
-                    const uint32_t c = cnt[j];
-                    sum += c;
-                    big = max(big, c);
+            // stable argsort; TSPJ's two segments one after the other
+            const int split = (kind == TSPJ) ? n / 2 : n;
+            const bool points = kind == TSP_COORDS || kind == BITSP_COORDS;
+            const bool want_perm = !points || L.perm_out;
+            bool sorted = true, summed = false;
+            if (points) {
+                // the tour's edges chunk by chunk.  TSP: edge e joins stops e and e + 1, the last the
+                // first; bi-objective: from the depot (point 0), edge e joins stops e - 1 and e, back to
+                // the depot
+                const bool open = kind == BITSP_COORDS;
+                const int objs = open ? 2 : 1;
+                float acc[2] = {0.0f, 0.0f};
+                float2 head[2], last[2];
+                float2* pt = reinterpret_cast<float2*>(row_scratch(s, kBigChunk));
+                auto chunk = [&](int p0, int m) {
+                    if (want_perm)
+                        for (int p = t; p < m; p += BLOCK) perm[p0 + p] = (int)kin[s.perm[p]].y;
+                    for (int ob = 0; ob < objs; ++ob) {
+                        const float2* xy = reinterpret_cast<const float2*>(ob ? sd.xy2 : sd.xy);
+                        // the points by local index, all of a thread's fetches in flight
+                        constexpr int U = kBigChunk / BLOCK;
+                        {
+                            float2 f[U];
+#pragma unroll
+                            for (int u = 0; u < U; ++u) {
+                                const int x = t + u * BLOCK;
+                                if (x < m) f[u] = __ldg(xy + kin[x].y + (open ? 1 : 0));
+                            }
+#pragma unroll
+                            for (int u = 0; u < U; ++u)
+                                if (t + u * BLOCK < m) pt[t + u * BLOCK] = f[u];
+                        }
+                        __syncthreads();
+                        if (p0 == 0) {
+                            head[ob] = open ? __ldg(xy) : pt[s.perm[0]];
+                            last[ob] = head[ob];
+                        }
+                        const float2 before = last[ob];
+                        last[ob] = pt[s.perm[m - 1]];
+                        // the edge into position p0 + p: number p0 + p (open) or p0 + p - 1; the terms take
+                        // the places of the sorted keys
+                        const int e0 = p0 - (open ? 0 : 1);
+#pragma unroll 2
+                        for (int p = t; p < m; p += BLOCK)
+                            kin[p].x = __float_as_uint(edge_pts(p ? pt[s.perm[p - 1]] : before, pt[s.perm[p]]));
+                        __syncthreads();
+                        if (t < 256) {
+                            // lane t adds the terms whose number is t modulo 256, in order
+                            int p = (t - e0) & 255;
+                            for (; p < m; p += 256)
+                                if (e0 + p >= 0) acc[ob] = __fadd_rn(acc[ob], __uint_as_float(kin[p].x));
+                        }
+                        __syncthreads();
+                    }
+                };
+                sorted = long_argsort(row, n, reinterpret_cast<uint2*>(sc), s, kin, bins, first_bin, g, chunk);
+                if (sorted) {
+                    summed = true;
+                    for (int ob = 0; ob < objs; ++ob) {
+                        const int e = open ? n : n - 1;  // the edge back to the start
+                        if (t == (e & 255)) acc[ob] = __fadd_rn(acc[ob], edge_pts(last[ob], head[ob]));
+                        res[ob] = lane_tree(acc[ob], red_f, t);
+                    }
                 }
-                uint32_t run = block_exclusive_scan<BLOCK>(sum, warp_tot, nullptr);
-                for (int j = t * ch; j < t * ch + ch; ++j) {
-                    const uint32_t c = cnt[j];
-                    cnt[j] = run;
-                    run += c;
-                }
-                if (t == 0) cnt[NB] = (uint32_t)n;
-                heavy = __syncthreads_or(big > kHeavyBucket) != 0;
-            }
-            for (int i = t; i < n; i += BLOCK) {
-                const float k = row[i];
-                sc[cnt[bucket(k, i)] + (uint32_t)perm[i]] = ((unsigned long long)okey(k) << 32) | (uint32_t)i;
-            }
-            __syncthreads();
-            if (heavy) {
-                // equal or extreme keys in few buckets: sort each segment's composites
-                heavy_row_perm<BLOCK>(sc, perm, n, split);
             } else {
-                for (int i = t; i < n; i += BLOCK) {
-                    const float k = row[i];
-                    const int b = bucket(k, i);
-                    const uint32_t b0 = cnt[b], b1 = cnt[b + 1];
-                    const unsigned long long me = ((unsigned long long)okey(k) << 32) | (uint32_t)i;
-                    uint32_t rk = b0;
-                    for (uint32_t q = b0; q < b1; ++q) rk += (sc[q] < me) ? 1u : 0u;
-                    perm[rk] = i;
+                for (int i0 = 0; i0 < n && sorted; i0 += split) {
+                    const int m0 = (i0 == 0) ? split : n - split;
+                    sorted = long_argsort(row + i0, m0, reinterpret_cast<uint2*>(sc), s, kin, bins, first_bin, g,
+                                          [&](int p0, int m) {
+                                              for (int p = t; p < m; p += BLOCK)
+                                                  perm[i0 + p0 + p] = i0 + (int)kin[s.perm[p]].y;
+                                          });
                 }
             }
+            if (!sorted) {
+                // equal or extreme keys in few bins: the row's composites sorted in place
+                for (int i = t; i < n; i += BLOCK) sc[i] = ((unsigned long long)okey(row[i]) << 32) | (uint32_t)i;
+                __syncthreads();
+                heavy_row_perm<BLOCK>(sc, perm, n, split);
+            }
             __syncthreads();
-            for (int j = t; j <= NB; j += BLOCK) cnt[j] = 0u;  // for the next row
-            if (kind == TSP_COORDS) {
-                const float* xy = sd.xy;
-                canon_sum<BLOCK, 1>(n, [&](int e, float* d) {
-                    const int a = perm[e], b = perm[(e + 1 < n) ? e + 1 : 0];
-                    d[0] = edge_xy(xy, a, b);
-                }, red_f, res);
+            if (summed) {
+                // done with the order
+            } else if (kind == TSP_COORDS) {
+                const float2* xy = reinterpret_cast<const float2*>(sd.xy);
+                res[0] = long_tour<true>(n, perm, [&](const int* id, float* d) {
+                    float2 p[5];
+#pragma unroll
+                    for (int i = 0; i < 5; ++i) p[i] = __ldg(xy + id[i]);
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) d[i] = edge_pts(p[i], p[i + 1]);
+                }, ed, red_f, t);
             } else if (kind == TSP_MATRIX) {
                 const float* mat = sd.mat;
-                canon_sum<BLOCK, 1>(n, [&](int e, float* d) {
-                    const int a = perm[e], b = perm[(e + 1 < n) ? e + 1 : 0];
-                    d[0] = __ldg(mat + (size_t)a * n + b);
-                }, red_f, res);
-            } else if (kind == BITSP_COORDS) {
-                const float* xy0 = sd.xy;
-                const float* xy1 = sd.xy2;
-                canon_sum<BLOCK, 2>(n + 1, [&](int e, float* d) {
-                    const int a = (e == 0) ? 0 : perm[e - 1] + 1;
-                    const int b = (e == n) ? 0 : perm[e] + 1;
-                    d[0] = edge_xy(xy0, a, b);
-                    d[1] = edge_xy(xy1, a, b);
-                }, red_f, res);
-            } else if (kind == BITSP_MATRIX) {
-                const float* m0 = sd.mat;
-                const float* m1 = sd.mat2;
-                const size_t np1 = (size_t)n + 1;
-                canon_sum<BLOCK, 2>(n + 1, [&](int e, float* d) {
-                    const int a = (e == 0) ? 0 : perm[e - 1] + 1;
-                    const int b = (e == n) ? 0 : perm[e] + 1;
-                    d[0] = __ldg(m0 + (size_t)a * np1 + b);
-                    d[1] = __ldg(m1 + (size_t)a * np1 + b);
-                }, red_f, res);
+                res[0] = long_tour<true>(n, perm, [&](const int* id, float* d) {
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) d[i] = __ldg(mat + (size_t)id[i] * n + id[i + 1]);
+                }, ed, red_f, t);
+            } else if (kind == BITSP_COORDS || kind == BITSP_MATRIX) {
+                for (int ob = 0; ob < 2; ++ob) {
+                    const float2* xy = reinterpret_cast<const float2*>(ob ? sd.xy2 : sd.xy);
+                    const float* mat = ob ? sd.mat2 : sd.mat;
+                    res[ob] = long_tour<false>(n, perm, [&](const int* id, float* d) {
+                        if (kind == BITSP_COORDS) {
+                            float2 p[5];
+#pragma unroll
+                            for (int i = 0; i < 5; ++i) p[i] = __ldg(xy + id[i]);
+#pragma unroll
+                            for (int i = 0; i < 4; ++i) d[i] = edge_pts(p[i], p[i + 1]);
+                        } else {
+#pragma unroll
+                            for (int i = 0; i < 4; ++i) d[i] = __ldg(mat + (size_t)id[i] * (n + 1) + id[i + 1]);
+                        }
+                    }, ed, red_f, t);
+                }
             } else if (kind == KNAP_GREEDY) {
                 res[0] = knap_greedy<BLOCK>(perm, n, sd.wv, sd.capi, red_ll, misc, reinterpret_cast<int2*>(sc));
             } else if (kind == TSPJ) {
@@ -881,7 +1061,9 @@ cudaError_t launch_rows_global(const RowLaunch& L, int kind, int grid, cudaStrea
     if (kind == MOVRP) return cudaErrorInvalidValue;  // MO-VRP rows fit in shared memory only
     if (L.ntasks <= 0 || grid <= 0) return cudaSuccess;
     if (grid > L.ntasks) grid = L.ntasks;
-    row_kernel_big<<<grid, kBigBlock, 0, s>>>(L);
+    const cudaError_t e = raise_smem_limit(reinterpret_cast<const void*>(row_kernel_big), big_smem_bytes());
+    if (e != cudaSuccess) return e;
+    row_kernel_big<<<grid, kBigBlock, big_smem_bytes(), s>>>(L);
     return cudaGetLastError();
 }
 

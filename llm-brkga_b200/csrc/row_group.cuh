@@ -97,15 +97,23 @@ __device__ __forceinline__ int key_bucket(float key, float nbf, int nb) {
 // the same (key, index) order.
 constexpr int kWindow = 8, kHeavyKeys = 32;
 
+// what orders equal keys: the index itself, or the gene an index stands for (indices past the
+// last gene are padding)
+__device__ __forceinline__ uint32_t gene_of(const uint2* gene, int genes, uint16_t x) {
+    if (!gene) return x;
+    return (int)x < genes ? gene[x].y : 0xFFFFFFFFu;
+}
+
 template <int T>
-__device__ __noinline__ void sort_heavy_segment(int32_t* k, uint16_t* x, int n, int tid, int rg) {
+__device__ __noinline__ void sort_heavy_segment(int32_t* k, uint16_t* x, int n, int tid, int rg, const uint2* gene,
+                                                int genes) {
     RowGroup<T> g;
     g.tid = tid;
     g.rg = rg;
     auto order = [&](int i, int j) {
         const int32_t a = k[i], b = k[j];
         const uint16_t u = x[i], v = x[j];
-        if (b < a || (b == a && v < u)) {
+        if (b < a || (b == a && gene_of(gene, genes, v) < gene_of(gene, genes, u))) {
             k[i] = b, k[j] = a;
             x[i] = v, x[j] = u;
         }
@@ -132,19 +140,21 @@ __device__ __noinline__ void sort_heavy_segment(int32_t* k, uint16_t* x, int n, 
 
 // ranks by a loop over w neighbours on each side (buckets of kWindow + 2 .. kHeavyKeys keys)
 template <int T>
-__device__ __noinline__ void rank_loop(const int32_t* sk, const uint16_t* si, uint16_t* perm, int first, int count, int out0, int w, int tid) {
+__device__ __noinline__ void rank_loop(const int32_t* sk, const uint16_t* si, uint16_t* perm, int first, int count, int out0, int w, int tid,
+                                       const uint2* gene, int genes) {
     for (int q = tid; q < count; q += T) {
         const int32_t a = sk[first + q];
         const uint16_t x = si[first + q];
+        const uint32_t me = gene_of(gene, genes, x);
         int r = q;
         for (int d = 1; d <= w; ++d) {
             if (q >= d) {
                 const int32_t b = sk[first + q - d];
-                r -= (b > a || (b == a && si[first + q - d] > x)) ? 1 : 0;
+                r -= (b > a || (b == a && gene_of(gene, genes, si[first + q - d]) > me)) ? 1 : 0;
             }
             if (q + d < count) {
                 const int32_t b = sk[first + q + d];
-                r += (b < a || (b == a && si[first + q + d] < x)) ? 1 : 0;
+                r += (b < a || (b == a && gene_of(gene, genes, si[first + q + d]) < me)) ? 1 : 0;
             }
         }
         perm[out0 + r] = x;
@@ -152,13 +162,13 @@ __device__ __noinline__ void rank_loop(const int32_t* sk, const uint16_t* si, ui
 }
 
 // equal keys in a thread's window: the window took them in position order; by index instead
-static __device__ __noinline__ int tie_fix(const int32_t* sk, const uint16_t* si, int p) {
+static __device__ __noinline__ int tie_fix(const int32_t* sk, const uint16_t* si, int p, const uint2* gene, int genes) {
     const int32_t a = sk[p];
-    const uint16_t x = si[p];
+    const uint32_t me = gene_of(gene, genes, si[p]);
     int r = 0;
     for (int d = 1; d <= kWindow; ++d) {
-        if (sk[p - d] == a && si[p - d] > x) --r;
-        if (sk[p + d] == a && si[p + d] < x) ++r;
+        if (sk[p - d] == a && gene_of(gene, genes, si[p - d]) > me) --r;
+        if (sk[p + d] == a && gene_of(gene, genes, si[p + d]) < me) ++r;
     }
     return r;
 }
@@ -193,10 +203,11 @@ __device__ __forceinline__ void count_keys(const float4& k, int q, int split, co
     atomicAdd(&s.cnt[bucket_at<SPLIT>(k.w, 4 * q + 3, split, s.nb, bucket)], 1u);
 }
 
-// keys(q) returns keys 4 q .. 4 q + 3 as count_keys saw them
+// keys(q) returns keys 4 q .. 4 q + 3 as count_keys saw them; gene: what the indices stand for,
+// where equal keys go by that instead of the index
 template <int T, bool SPLIT, typename BucketF, typename KeysF>
 __device__ __forceinline__ void sort_row(int n, int split, const RowBuf& s, const RowGroup<T>& g, BucketF bucket,
-                                         KeysF keys) {
+                                         KeysF keys, const uint2* gene = nullptr, int genes = 0) {
     constexpr int NW = T / 32;
     const int t = g.tid, lane = t & 31, warp = t >> 5;
     g.sync();
@@ -277,12 +288,12 @@ __device__ __forceinline__ void sort_row(int n, int split, const RowBuf& s, cons
     const int w = (int)big - 1;
     if (w > kWindow) {
         if (big > (uint32_t)kHeavyKeys) {
-            sort_heavy_segment<T>(s.sk, s.si, gap0, t, g.rg);
-            if (SPLIT) sort_heavy_segment<T>(s.sk + seg1, s.si + seg1, n - split, t, g.rg);
+            sort_heavy_segment<T>(s.sk, s.si, gap0, t, g.rg, gene, genes);
+            if (SPLIT) sort_heavy_segment<T>(s.sk + seg1, s.si + seg1, n - split, t, g.rg, gene, genes);
             for (int p = t; p < n; p += T) s.perm[p] = s.si[p < gap0 ? p : p + shift];
         } else {
-            rank_loop<T>(s.sk, s.si, s.perm, 0, gap0, 0, w, t);
-            if (SPLIT) rank_loop<T>(s.sk, s.si, s.perm, seg1, n - split, split, w, t);
+            rank_loop<T>(s.sk, s.si, s.perm, 0, gap0, 0, w, t, gene, genes);
+            if (SPLIT) rank_loop<T>(s.sk, s.si, s.perm, seg1, n - split, split, w, t, gene, genes);
         }
         g.sync();
         return;
@@ -327,7 +338,7 @@ __device__ __forceinline__ void sort_row(int n, int split, const RowBuf& s, cons
         }
         if (tie) {
 #pragma unroll
-            for (int i = 0; i < 4; ++i) r[i] += tie_fix(s.sk, s.si, 4 * c + i);
+            for (int i = 0; i < 4; ++i) r[i] += tie_fix(s.sk, s.si, 4 * c + i, gene, genes);
         }
         const uint32_t x[4] = {x2.x & 0xFFFFu, x2.x >> 16, x2.y & 0xFFFFu, x2.y >> 16};
 #pragma unroll
@@ -354,6 +365,8 @@ __device__ __forceinline__ void zero_counters(const RowBuf& s, int tid) {
 // ---------------------------------------------------------------------------------------
 // fitness
 // ---------------------------------------------------------------------------------------
+// Euclidean edge exactly as the reference builds its matrix (configs/tsp_config.hpp:366-368):
+// float dx, dy; sqrt(dx*dx + dy*dy), no contraction, correctly rounded sqrt
 __device__ __forceinline__ float edge_pts(float2 pa, float2 pb) {
     const float dx = __fsub_rn(pa.x, pb.x);
     const float dy = __fsub_rn(pa.y, pb.y);

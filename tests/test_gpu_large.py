@@ -124,3 +124,22 @@ def test_batch_rejects_rows_beyond_shared_memory(cuda):
         B().Batch([pb], [B().params(16, 3, 2, 0.7, 5, seed=1)])
     assert ei.value.code == -6
     assert "brkga_create" in str(ei.value)
+
+
+@pytest.mark.parametrize("n", [14000, 20481, 131073, 150001])
+@pytest.mark.parametrize("shape", ["flat", "skewed", "tied", "edge"])
+def test_chunked_sort_large(cuda, n, shape):
+    """the two-level sort: chunks picked out of the row (up to 12) and dealt through scratch
+    (more), bins near half a chunk and past it (sorted as a whole), equal keys across bins"""
+    rng = np.random.default_rng(n)
+    k = rng.random((2, n))
+    if shape == "skewed":
+        k = k ** 8
+    elif shape == "tied":
+        k = np.floor(k * 3000) / 3000
+    elif shape == "edge":
+        k[0, :5119] = 0.25 + rng.random(5119) / 8192  # one bin of 4096, one key below half a chunk
+        k[1, :5200] = 0.75 + rng.random(5200) / 8192
+    keys = k.astype(np.float32)
+    xy = I.tsp_coords(n, seed=n)
+    check_tsp(B().tsp(xy), O.OracleProblem(O.TSP_COORDS, n, xy=xy), keys, cuda)
