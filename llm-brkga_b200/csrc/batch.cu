@@ -254,6 +254,8 @@ static int32_t pull_state(Group& g) {
     cudaError_t e = cudaStreamSynchronize(g.stream);
     if (e == cudaSuccess) e = cudaMemcpy(g.hd.data(), g.dd, sizeof(PopDesc) * nd, cudaMemcpyDeviceToHost);
     if (e != cudaSuccess) return cuda_fail(e, "descriptor read-back");
+    for (const PopDesc& d : g.hd)
+        if (d.stuck) return fail(BRKGA_ERR_TIMEOUT, "a wait between the launch's CTAs ran out; the populations are not valid");
     for (Member* m : g.members)
         for (int i = 0; i < m->ndesc; ++i) m->pop.hd_template[i] = g.hd[m->first + i];
     return BRKGA_OK;

@@ -154,7 +154,8 @@ struct PopDesc {
     int32_t advanced;
     // TSPJ random 2-opt local search period (0 = off)
     int32_t ls_interval;
-    int32_t stuck;            // a bounded wait of an evolve launch ran out
+    int32_t stuck;            // a bounded wait between a launch's CTAs ran out
+    int32_t* stuck_host;      // pinned copy of it for a call that reads no descriptor back, or null
 };
 
 __host__ __device__ __forceinline__ bool at_limit(const PopDesc& d) { return d.gen_limit != 0u && d.gen >= d.gen_limit; }

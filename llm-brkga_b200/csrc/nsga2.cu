@@ -739,15 +739,24 @@ __device__ __forceinline__ bool select_active(const PopDesc& d, int mode) {
 
 // Ranks by peeling, on one thread-block cluster per population.  A point's dominator row
 // stays in registers for the whole peel: eight lanes hold it, 4 WL bytes each, and a warp
-// 16 points.  A front is a bit mask of the points in it; a point's count of dominators left
-// drops by the population count of (its row and the front), doubled for the first front
-// (its points are listed twice); points at or below zero form the next front.  Each warp
-// sends its 16 bits of the next front into every CTA's shared memory, and one cluster
-// barrier a front completes the mask.  Nothing is merged across warps: summing the rows of a
-// front's members column by column instead (bit-sliced partial sums of eight warps, added in
-// sequence, then subtracted) took about 6 us a front at N = 4096.  Population counts issue
-// at a quarter of the rate of logic, so a lane's words are first added carry-save (16 words:
-// 5 counts).
+// 16 points.  Mask k holds the points of the fronts 0..k; a point joins front k + 1 when its
+// dominators outside the mask are no more than those of the first front (whose points are
+// listed twice, so that each takes two off the count).
+//
+// A front is a chain: counts, the CTA's 256 bits gathered, the exchange, the mask's size.
+//  - A CTA sends its words to every CTA with st.async, which completes on the receiver's
+//    mbarrier: 650 cycles a front for 16 CTAs, where 16-bit stores by every warp and a cluster
+//    barrier took 1900 and one warp's stores and a cluster barrier 1300.  Four masks go round:
+//    a CTA sends mask k + 3 only after every other CTA has sent mask k + 2, and none does
+//    before it is done reading masks k - 1 and k.
+//  - A step (four points) is counted only if one of its points can come to zero: its count less
+//    the points that joined since it was last counted.  About half the steps of a front are.
+//  - Counts are bound by logic (two cycles a warp) and population counts (eight): 16 words take
+//    6 full adders and 10 counts, about equal shares.
+// Measured, NSGA-II generations of 4096-point pools (7 fronts) and 3000-point pools (15 to 19
+// fronts): 67.3 -> 64.8 and 56.0 -> 51.6 us a generation; the ranks of 4096 points in all fronts
+// and their crowding 94.4 -> 86.8 us.  (Merging the rows of a front's members by column instead,
+// bit-sliced, took about 6 us a front at N = 4096.)
 //
 // The pool of a generation (mode 0) is peeled only up to the front where the survivors
 // (rank-0 points counted twice) first exceed P: that front is cut by crowding, and no
@@ -756,46 +765,68 @@ __device__ __forceinline__ bool select_active(const PopDesc& d, int mode) {
 // generation are the same as with every front peeled.  Ranks -> domcnt[0, N).
 constexpr int kPeelThreads = 512, kPeelWarpPoints = 16, kPeelPoints = kPeelThreads / 32 * kPeelWarpPoints;
 
-// set bits of x[0, n) (n = 4, 8 or 16): carry-save adders, then a count per weight
+// set bits of x[0, n) (n = 4, 8 or 16): full adders until the logic (two cycles a warp) takes
+// about as long as the counts left (eight cycles a warp)
 template <int n>
 __device__ __forceinline__ int count_bits(const uint32_t (&x)[n]) {
-    uint32_t one = 0u, two = 0u, four = 0u, eight = 0u;
-    int high = 0;
+    int one = 0, two = 0;
     auto add3 = [](uint32_t& s, uint32_t b, uint32_t c) {  // s <- the sum bit; returns the carry
         const uint32_t cy = (s & b) | (c & (s | b));
         s = s ^ b ^ c;
         return cy;
     };
+    auto add7 = [&](uint32_t a, uint32_t b, uint32_t c, uint32_t d, uint32_t e, uint32_t f, uint32_t g) {
+        two += __popc(add3(a, b, c)) + __popc(add3(d, e, f));
+        two += __popc(add3(a, d, g));
+        return a;
+    };
+    if constexpr (n == 4) {
+        uint32_t a = x[0];
+        two = __popc(add3(a, x[1], x[2]));
+        one = __popc(a) + __popc(x[3]);
+    } else {
 #pragma unroll
-    for (int i = 0; i < n; i += 4) {
-        const uint32_t t0 = add3(one, x[i], x[i + 1]), t1 = add3(one, x[i + 2], x[i + 3]);
-        const uint32_t f = add3(two, t0, t1);
-        const uint32_t e = four & f;
-        four ^= f;
-        const uint32_t s16 = eight & e;
-        eight ^= e;
-        if (i == 12) high = 16 * __popc(s16);
+        for (int i = 0; i < n; i += 8)
+            one += __popc(add7(x[i], x[i + 1], x[i + 2], x[i + 3], x[i + 4], x[i + 5], x[i + 6])) + __popc(x[i + 7]);
     }
-    int c = __popc(one) + 2 * __popc(two) + 4 * __popc(four);
-    if (n > 4) c += 8 * __popc(eight);
-    return c + high;
+    return one + 2 * two;
 }
+
+__device__ __forceinline__ uint32_t shared_addr(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
+
+constexpr uint32_t kMaskPolls = 1u << 24;  // polls of one wait: most of a second; a front is microseconds
 
 template <int WL>
 __global__ void __launch_bounds__(kPeelThreads, 1) nsga_peel_rows_kernel(PopDesc* dd, int mode) {
     dep_wait();
     namespace cg = cooperative_groups;
-    constexpr int NW = 8 * WL;  // words of a front mask
-    __shared__ __align__(16) uint32_t F[2][NW];  // front k in F[k & 1]
+    constexpr int NW = 8 * WL;  // words of a mask
+    __shared__ __align__(16) uint32_t F[4][NW];  // the points of the fronts 0..k in F[k & 3]
+    __shared__ __align__(16) uint16_t out[kPeelThreads / 32];  // the CTA's part of the next mask
+    __shared__ __align__(8) uint64_t bar[4];  // of each mask: every CTA's part has arrived
     cg::cluster_group cluster = cg::this_cluster();
     const int csize = (int)cluster.num_blocks(), crank = (int)cluster.block_rank();
     PopDesc& d = dd[blockIdx.x / csize];
     if (!select_active(d, mode)) return;  // the same decision in every CTA of the cluster
     const int N = (mode == 0) ? 2 * d.P : d.P;
-    const int W = (N + 31) / 32, Wmax = d.domW;
+    const int Wmax = d.domW;
     const int t = threadIdx.x, lane = t & 31, warp = t >> 5, sub = lane & 7;
-    const int p0 = crank * kPeelPoints + warp * kPeelWarpPoints;  // the warp's points; step s: p0 + 4 s + lane / 8
+    // A CTA has pairs of words (64 points each) from the four quarters of the points: a pool's
+    // survivors come in the order of their last fronts, so neighbours are at work together.
+    auto word_of = [&](int quarter) { return 2 * (quarter * csize + crank); };
+    const int word = word_of(warp / 4) + ((warp >> 1) & 1);
+    const int p0 = 32 * word + kPeelWarpPoints * (warp & 1);  // the warp's points; step s: p0 + 4 s + lane / 8
 
+    if (t < 4) {
+        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(shared_addr(&bar[t])) : "memory");
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    // (Words past N stay zero in the masks: rows may hold anything there.)
+    for (int w = t; w < NW; w += kPeelThreads) {
+        F[1][w] = (w < N / 32) ? 0xFFFFFFFFu : (w == N / 32 && (N & 31)) ? (1u << (N & 31)) - 1u : 0u;
+        F[0][w] = F[2][w] = F[3][w] = 0u;
+    }
+    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
     uint32_t x[4][WL];
 #pragma unroll
     for (int st = 0; st < 4; ++st) {
@@ -808,23 +839,22 @@ __global__ void __launch_bounds__(kPeelThreads, 1) nsga_peel_rows_kernel(PopDesc
             x[st][4 * c] = v.x, x[st][4 * c + 1] = v.y, x[st][4 * c + 2] = v.z, x[st][4 * c + 3] = v.w;
         }
     }
-    // counts of the points' dominators in the mask F[b], two per packed pair: steps 0 | 1, 2 | 3
-    auto dominators_in = [&](int b, int (&cnt)[4]) {
+    // counts of the points' dominators in a mask, for the steps in `act` (0 for the others)
+    auto dominators_in = [&](const uint32_t* f, uint32_t act, int (&cnt)[4]) {
         uint32_t m[WL];
 #pragma unroll
         for (int c = 0; c < WL / 4; ++c) {
-            const uint4 v = *reinterpret_cast<const uint4*>(&F[b][32 * c + 4 * sub]);
+            const uint4 v = *reinterpret_cast<const uint4*>(f + 32 * c + 4 * sub);
             m[4 * c] = v.x, m[4 * c + 1] = v.y, m[4 * c + 2] = v.z, m[4 * c + 3] = v.w;
         }
-        uint32_t pk[2];
+        uint32_t pk[2] = {0u, 0u};  // two steps a word
 #pragma unroll
         for (int st = 0; st < 4; ++st) {
+            if (!((act >> st) & 1u)) continue;
             uint32_t y[WL];
 #pragma unroll
             for (int u = 0; u < WL; ++u) y[u] = x[st][u] & m[u];
-            const uint32_t c = (uint32_t)count_bits<WL>(y);
-            if (st & 1) pk[st >> 1] |= c << 16;
-            else pk[st >> 1] = c;
+            pk[st >> 1] |= (uint32_t)count_bits<WL>(y) << (16 * (st & 1));
         }
 #pragma unroll
         for (int o = 1; o < 8; o <<= 1) {
@@ -834,91 +864,144 @@ __global__ void __launch_bounds__(kPeelThreads, 1) nsga_peel_rows_kernel(PopDesc
         cnt[0] = (int)(pk[0] & 0xFFFFu), cnt[1] = (int)(pk[0] >> 16);
         cnt[2] = (int)(pk[1] & 0xFFFFu), cnt[3] = (int)(pk[1] >> 16);
     };
-    // the warp's points at or below zero and not ranked yet, as 16 bits, into every CTA's mask
-    uint32_t ranked = 0u;  // bit 4 s + lane / 8
-    auto send_front = [&](int b, const int (&cnt)[4]) {
+    uint32_t ranked = 0u, mine = 0u;  // the warp's points in the fronts so far, in the next one: bit 4 s + lane / 8
+    // points of the steps `act` at or below zero and not ranked yet join the next front: the
+    // CTA's 256 bits of mask b gathered, then sent to every CTA
+    auto send_front = [&](int b, uint32_t act, const int (&left)[4]) {
         uint32_t bits = 0u;
+        if (act) {
 #pragma unroll
-        for (int st = 0; st < 4; ++st) {
-            const uint32_t v = __ballot_sync(0xffffffffu, cnt[st] <= 0 && p0 + 4 * st + (lane >> 3) < N);
-            bits |= ((v & 1u) | ((v >> 7) & 2u) | ((v >> 14) & 4u) | ((v >> 21) & 8u)) << (4 * st);
+            for (int st = 0; st < 4; ++st) {
+                const uint32_t v =
+                    __ballot_sync(0xffffffffu, ((act >> st) & 1u) && left[st] <= 0 && p0 + 4 * st + (lane >> 3) < N);
+                bits |= ((v & 1u) | ((v >> 7) & 2u) | ((v >> 14) & 4u) | ((v >> 21) & 8u)) << (4 * st);
+            }
         }
-        bits &= ~ranked;
-        if (lane < csize)
-            reinterpret_cast<uint16_t*>(cluster.map_shared_rank(&F[b][0], lane))[p0 / kPeelWarpPoints] = (uint16_t)bits;
+        mine = bits & ~ranked;
+        ranked |= mine;
+        if (lane == 0) out[warp] = (uint16_t)ranked;
+        __syncthreads();
+        if (t < 4 * csize) {  // one pair of words to one CTA
+            const int q = t & 3;
+            const uint32_t to = shared_addr(&F[b][word_of(q)]), at = shared_addr(&bar[b]);
+            if (t == 0)
+                asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(at), "r"(32 * csize) : "memory");
+            const uint2 v = reinterpret_cast<const uint2*>(out)[q];
+            uint32_t rto, rat;
+            asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(rto) : "r"(to), "r"(t >> 2));
+            asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(rat) : "r"(at), "r"(t >> 2));
+            asm volatile("st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.v2.b32 [%0], {%1, %2}, [%3];"
+                         ::"r"(rto), "r"(v.x), "r"(v.y), "r"(rat)
+                         : "memory");
+        }
     };
-    // every point: the counts of all dominators.  (Words past N stay zero: rows may hold anything
-    // there, and no CTA writes them when the cluster covers fewer points than the mask.)
-    for (int w = t; w < NW; w += kPeelThreads) {
-        F[1][w] = (w < N / 32) ? 0xFFFFFFFFu : (w == N / 32 && (N & 31)) ? (1u << (N & 31)) - 1u : 0u;
-        F[0][w] = 0u;
-    }
-    cluster.sync();
-    int left[4];
-    dominators_in(1, left);
-    send_front(0, left);
-    cluster.sync();
-    if (csize * kPeelPoints < 32 * NW)
-        for (int w = csize * (kPeelPoints / 32) + t; w < NW; w += kPeelThreads) F[1][w] = 0u;
+    // front k's mask is complete; false (in every thread of the CTA) when a wait ran out
+    auto await_front = [&](int k) {
+        const uint32_t at = shared_addr(&bar[k & 3]), parity = (uint32_t)(k >> 2) & 1u;
+        uint32_t done = 0u;
+        for (uint32_t n = 0; n < kMaskPolls && !done; ++n)
+            asm volatile(
+                "{.reg .pred p;\n\t"
+                "mbarrier.test_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\t"
+                "selp.u32 %0, 1, 0, p;}"
+                : "=r"(done)
+                : "r"(at), "r"(parity)
+                : "memory");
+        return __syncthreads_and((int)done) != 0;
+    };
     __syncthreads();
+    int need[4];  // every point: all its dominators, and once those of the first front are known, them once more
+    dominators_in(F[1], 15u, need);
+    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");  // every CTA's masks and barriers are set up
+    send_front(0, 15u, need);
 
     int survivors = 0, rest = 0, start = 0;
+    int reach[4] = {0, 0, 0, 0};  // listed points at which a step's points may come to zero
     // thread 0 of the cluster's first CTA records the front table (start of each front in
     // rank order, the cut front) for the grid-wide crowding and placement of mode 0
     int32_t* const ft = (crank == 0 && t == 0) ? d.nft : nullptr;
+    bool stuck = false;
     for (int k = 0;; ++k) {
-        const uint32_t* f = F[k & 1];
-        // the front's size, and the members before this warp's points
-        const int word = p0 / 32;
-        int total = 0, pre = 0;
-#pragma unroll
-        for (int c = 0; c < (NW + 31) / 32; ++c) {
-            const int w = 32 * c + lane;
-            const int pc = (w < W) ? __popc(f[w]) : 0;
-            total += pc;
-            pre += (w < word) ? pc : 0;
+        const uint32_t* const f = F[k & 3];
+        if (!await_front(k)) {
+            stuck = true;
+            break;
         }
-        const int nf = __reduce_add_sync(0xffffffffu, total);
-        if (nf == 0) {  // every CTA sees the same front
+        int total = 0;  // points of the fronts 0..k
+#pragma unroll
+        for (int c = 0; c < NW / 32; ++c) total += __popc(f[32 * c + lane]);
+        total = __reduce_add_sync(0xffffffffu, total);
+        const int nf = total - start;  // every CTA sees the same front
+        survivors += (k == 0) ? 2 * nf : nf;
+        const bool cut = mode == 0 && nf > 0 && survivors > d.P;
+        const uint32_t members = mine;
+        if (nf > 0 && !cut) {
+            // the steps with a point that may come to zero with this front
+            uint32_t act = 0u;
+#pragma unroll
+            for (int st = 0; st < 4; ++st)
+                act |= __any_sync(0xffffffffu, reach[st] <= total && !((ranked >> (4 * st + (lane >> 3))) & 1u)) ? 1u << st : 0u;
+            int left[4] = {1, 1, 1, 1};
+            if (act) {
+                int cnt[4];
+                dominators_in(f, act, cnt);
+#pragma unroll
+                for (int st = 0; st < 4; ++st) {
+                    if (!((act >> st) & 1u)) continue;
+                    if (k == 0) need[st] -= cnt[st];
+                    left[st] = need[st] - cnt[st];
+                    reach[st] = (p0 + 4 * st + (lane >> 3) < N) ? left[st] + total : INT_MAX;
+                }
+            }
+            send_front((k + 1) & 3, act, left);
+        }
+        // while the next mask is on its way: the ranks of the warp's members of front k, and
+        // their places in the list of fronts
+        if (ft) ft[2 + k] = start;
+        if (members) {
+            const uint32_t* const before = F[(k + 3) & 3];  // fronts 0..k - 1
+            int pre = 0;
+#pragma unroll
+            for (int c = 0; c < NW / 32; ++c) {
+                const int w = 32 * c + lane;
+                const uint32_t v = (k == 0) ? f[w] : f[w] & ~before[w];
+                pre += (w < word) ? __popc(v) : (w == word && (warp & 1)) ? __popc(v & 0xFFFFu) : 0;
+            }
+            pre = __reduce_add_sync(0xffffffffu, pre);
+            if (lane < 16 && ((members >> lane) & 1u)) {
+                d.domcnt[p0 + lane] = k;
+                if (d.nlist) d.nlist[start + pre + __popc(members & ((1u << lane) - 1u))] = p0 + lane;
+            }
+        }
+        start = total;
+        if (nf == 0) {
             if (ft) {
                 ft[0] = k;
                 ft[1] = -1;
-                ft[2 + k] = start;
             }
             break;
         }
-        if (ft) ft[2 + k] = start;
-        const uint32_t mine = reinterpret_cast<const uint16_t*>(f)[p0 / kPeelWarpPoints];
-        if (mine) {  // the warp's members: their ranks, and their places in the list of fronts
-            pre = __reduce_add_sync(0xffffffffu, pre) + ((p0 & 16) ? __popc(f[word] & 0xFFFFu) : 0);
-            if (lane < 16 && ((mine >> lane) & 1u)) {
-                d.domcnt[p0 + lane] = k;
-                if (d.nlist) d.nlist[start + pre + __popc(mine & ((1u << lane) - 1u))] = p0 + lane;
+        if (cut) {
+            rest = k + 1;
+            if (ft) {  // the cut front k, then the points left as one last front
+                ft[1] = k;
+                ft[3 + k] = start;
+                ft[4 + k] = N;
+                ft[0] = (start < N) ? k + 2 : k + 1;
             }
-            ranked |= mine;
+            break;
         }
-        start += nf;
-        if (mode == 0) {
-            survivors += (k == 0) ? 2 * nf : nf;
-            if (survivors > d.P) {
-                rest = k + 1;
-                if (ft) {  // the cut front k, then the points left as one last front
-                    ft[1] = k;
-                    ft[3 + k] = start;
-                    ft[4 + k] = N;
-                    ft[0] = (start < N) ? k + 2 : k + 1;
-                }
-                break;
-            }
-        }
-        int dec[4];
-        dominators_in(k & 1, dec);
-#pragma unroll
-        for (int st = 0; st < 4; ++st) left[st] -= (k == 0) ? 2 * dec[st] : dec[st];
-        send_front((k + 1) & 1, left);
-        cluster.sync();
+    }
+    __syncwarp();
+    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+    if (stuck && t == 0) {
+        d.stuck = 1;
+        if (d.stuck_host) *d.stuck_host = 1;
     }
     if (lane < 16 && p0 + lane < N && !((ranked >> lane) & 1u)) d.domcnt[p0 + lane] = rest;
+    // no CTA leaves while another may still send to it
+    __syncwarp();
+    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
 
 using PeelFn = void (*)(PopDesc*, int);
@@ -1630,6 +1713,7 @@ static int32_t read_desc(NsgaState& s, cudaStream_t st, PopDesc* d) {
     cudaError_t e = cudaStreamSynchronize(st);
     if (e == cudaSuccess) e = cudaMemcpy(d, s.dd, sizeof(PopDesc), cudaMemcpyDeviceToHost);
     if (e != cudaSuccess) return cuda_fail(e, "descriptor read-back");
+    if (d->stuck) return fail(BRKGA_ERR_TIMEOUT, "a wait between the launch's CTAs ran out; the population is not valid");
     return BRKGA_OK;
 }
 
@@ -1784,11 +1868,20 @@ static int32_t static_scratch(uint32_t** out) {
 // scratch of the operator entry points (grow-only, per device)
 static std::mutex g_op_mu;
 static std::map<int, std::pair<void*, size_t>> g_op_buf;
+static int32_t* g_op_stuck = nullptr;  // pinned: a wait in an operator's kernel ran out (read without a copy)
 
 static int32_t op_scratch(size_t need, void** out) {
     int dev = 0;
     cudaError_t e = cudaGetDevice(&dev);
     if (e != cudaSuccess) return cuda_fail(e, "cudaGetDevice");
+    if (!g_op_stuck) {
+        if ((e = cudaHostAlloc(&g_op_stuck, sizeof(int32_t), cudaHostAllocPortable | cudaHostAllocMapped)) != cudaSuccess) {
+            g_op_stuck = nullptr;
+            cudaGetLastError();
+            return fail(BRKGA_ERR_OOM, std::string("operator flag: ") + cudaGetErrorString(e));
+        }
+        *g_op_stuck = 0;
+    }
     auto& b = g_op_buf[dev];
     if (b.second < need) {
         if (b.first) {
@@ -1854,6 +1947,7 @@ int32_t brkga_pareto_rank_bitmatrix(const float* d_obj, int32_t N, int32_t m, in
         hd.domS = a.S;
         hd.domW = W;
         hd.domcnt = d_rank;
+        hd.stuck_host = g_op_stuck;
         PopDesc* dd = reinterpret_cast<PopDesc*>((char*)buf + doff);
         if ((e = cudaMemcpyAsync(dd, &hd, sizeof(hd), cudaMemcpyHostToDevice, st)) != cudaSuccess)
             return cuda_fail(e, "peel descriptor");
@@ -1867,6 +1961,10 @@ int32_t brkga_pareto_rank_bitmatrix(const float* d_obj, int32_t N, int32_t m, in
     }
     // the scratch is shared by later calls: finish before returning
     if ((e = cudaStreamSynchronize(st)) != cudaSuccess) return cuda_fail(e, "peel");
+    if (*static_cast<volatile int32_t*>(g_op_stuck)) {
+        *g_op_stuck = 0;
+        return fail(BRKGA_ERR_TIMEOUT, "a wait between the peel's CTAs ran out; the ranks are not valid");
+    }
     return BRKGA_OK;
 }
 
