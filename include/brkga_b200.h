@@ -198,8 +198,9 @@ int32_t brkga_local_search(brkga_problem* pb, float* d_pop, float* d_fitness, in
 int32_t brkga_pareto_rank(const float* d_obj, int32_t N, int32_t m, int32_t* d_rank, void* stream);
 /* The same ranks through the bit-packed dominance matrix for any m: bit j of row i set when
  * point i dominates point j, built 32 columns per __ballot_sync; fronts peeled by
- * bit-sliced column sums of the front's rows (for N <= 4096 on a cluster of eight CTAs,
- * the front exchanged through distributed shared memory).  Uses an internal device scratch
+ * bit-sliced column sums of the front's rows.  Up to 4096 points the rows hold the
+ * dominators (bit j: j dominates i) and stay in the registers of a cluster of up to 16
+ * CTAs, which exchange the front through distributed shared memory.  Uses an internal device scratch
  * of about N*ceil(N/32)*4 bytes and returns after the ranks are written. */
 int32_t brkga_pareto_rank_bitmatrix(const float* d_obj, int32_t N, int32_t m, int32_t* d_rank, void* stream);
 /* Pareto ranks exactly like brkga_pareto_rank, but the call allocates no device memory:

@@ -2,9 +2,11 @@
 // the reference's run / evolve_generation / get_best_individual surface.
 //
 // The population, its fitness, the rank order and the best-fitness history stay in HBM
-// for the whole run; one generation is two launches (the fused row kernel and the
-// elite-partition sort) that read their state from device-resident descriptors, so the
-// sequence is captured once as a CUDA graph and replayed.
+// for the whole run.  One single-objective population evolves many generations in one
+// cooperative launch (evolve.cu).  Islands, two objectives and long rows take launches per
+// generation (the row kernel, then the elite partition or the NSGA-II selection) that read
+// their state from device-resident descriptors, so the sequence is captured once as a CUDA
+// graph and replayed.
 #include <algorithm>
 #include <cmath>
 #include <cstring>

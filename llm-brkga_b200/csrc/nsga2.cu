@@ -11,11 +11,11 @@
 // as two adjacent entries, and its survivor list takes first-front points twice.  All
 // three are reproduced here (ties fixed by index), bit for bit against the oracle.
 //
-// Ranks: bit-packed dominance matrix + bit-sliced front peeling (below).
-// Crowding: per objective a bitonic sort of (rank, objective, index) makes every front a
-// contiguous ordered run; each entry adds (next - prev) / range in list order.
-// Survivors: bitonic sort of the entry list (first-front points twice) by (rank, last
-// objective or -crowding for the front that is cut, index, copy); the first P entries.
+// Ranks: bit-packed dominator rows, peeled front by front on a thread-block cluster.
+// Crowding: each point's place, neighbours and extremes in its front in both objective
+// orders, by counting; each entry adds (next - prev) / range in list order.
+// Survivors: the entries (first-front points twice) by (rank, last objective or -crowding
+// for the front that is cut, index, copy); the first P of them.
 #include <algorithm>
 #include <cfloat>
 #include <map>
