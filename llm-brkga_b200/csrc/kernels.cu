@@ -458,7 +458,7 @@ __device__ __forceinline__ bool long_argsort(const float* key, int n, uint2* sc,
         if (m == 0) continue;
         const float lo = (float)b0, scale = __fdiv_rn((float)s.nb, (float)(b1 - b0));
         // monotone over the chunk's key range
-        auto bucket = [&](float k, int nb) {
+        auto bucket = [lo, scale](float k, int nb) {
             const float f = __fmul_rn(__fsub_rn(__fmul_rn(k, (float)kBigBins), lo), scale);
             return max((int)fminf(f, (float)nb - 1.0f), 0);
         };

@@ -337,7 +337,7 @@ __device__ __forceinline__ void row_work(const RowLaunch& L, const PopDesc& sd, 
         // 2. the visiting order: values span about [hb, hb + 1 + n * 1e-5], and any
         //    non-decreasing bucket map gives the same (value, index) order
         const float inv = __frcp_rn(__fadd_rn(1.0f, __fmul_rn((float)n, 1.0e-5f)));
-        auto shifted = [&](float v, int nb) { return key_bucket(__fmul_rn(__fsub_rn(v, hb), inv), (float)nb, nb); };
+        auto shifted = [hb, inv](float v, int nb) { return key_bucket(__fmul_rn(__fsub_rn(v, hb), inv), (float)nb, nb); };
         for (int q = t; 4 * q < n; q += T) {
             float4 k = kin[q];
             const float f = (float)(4 * q);

@@ -91,10 +91,10 @@ __device__ __forceinline__ int key_bucket(float key, float nbf, int nb) {
 }
 
 // A bucket's keys are ranked against their neighbours, so equal keys, keys outside [0, 1)
-// and NaNs (few buckets) cost the square of the largest bucket.  Up to kWindow + 1 keys a
-// bucket take the window below (nearly every row of keys in [0, 1)), up to kHeavyKeys a
-// loop, and rows beyond that an ascending bitonic network: O(n log^2 n) on any input, and
-// the same (key, index) order.
+// and NaNs (few buckets) cost the square of the bucket.  Up to kWindow + 1 keys a
+// bucket take the window below (nearly every row of random keys in [0, 1)), up to kHeavyKeys a
+// loop over each key's bucket, and rows beyond that an ascending bitonic network:
+// O(n log^2 n) on any input, and the same (key, index) order.
 constexpr int kWindow = 8, kHeavyKeys = 32;
 
 // what orders equal keys: the index itself, or the gene an index stands for (indices past the
@@ -138,27 +138,42 @@ __device__ __noinline__ void sort_heavy_segment(int32_t* k, uint16_t* x, int n, 
     }
 }
 
-// ranks by a loop over w neighbours on each side (buckets of kWindow + 2 .. kHeavyKeys keys)
-template <int T>
-__device__ __noinline__ void rank_loop(const int32_t* sk, const uint16_t* si, uint16_t* perm, int first, int count, int out0, int w, int tid,
-                                       const uint2* gene, int genes) {
-    for (int q = tid; q < count; q += T) {
-        const int32_t a = sk[first + q];
-        const uint16_t x = si[first + q];
-        const uint32_t me = gene_of(gene, genes, x);
-        int r = q;
-        for (int d = 1; d <= w; ++d) {
-            if (q >= d) {
-                const int32_t b = sk[first + q - d];
-                r -= (b > a || (b == a && gene_of(gene, genes, si[first + q - d]) > me)) ? 1 : 0;
-            }
-            if (q + d < count) {
-                const int32_t b = sk[first + q + d];
-                r += (b < a || (b == a && gene_of(gene, genes, si[first + q + d]) < me)) ? 1 : 0;
-            }
+// Ranks by a loop over each key's own bucket: rows with a bucket of kWindow + 2 .. kHeavyKeys
+// keys.  Populations that have converged are full of them (keys that were selected lie close
+// together), so a row must not pay for its largest bucket at every key: over as many
+// neighbours as that bucket holds, a generation of a converged population (n = 1000, P = 2048)
+// took 48.8 us.  cnt holds the buckets' ends and is overwritten by the permutation, so the
+// ranks wait in local memory.
+constexpr int kMaxGroups = 16;  // a thread's keys at most, by four
+
+template <int T, bool SPLIT, typename BucketF>
+__device__ __noinline__ void rank_buckets(const int32_t* sk, const uint16_t* si, const uint32_t* cnt, uint16_t* perm, int n,
+                                          int split, int shift, int nb, BucketF bucket, int tid, int rg,
+                                          const uint2* gene, int genes) {
+    RowGroup<T> g;
+    g.tid = tid;
+    g.rg = rg;
+    const int nbs = SPLIT ? nb / 2 : nb;
+    uint16_t rank[4 * kMaxGroups];
+#pragma unroll 1
+    for (int q = tid, j = 0; q < n; q += T, ++j) {
+        const bool second = SPLIT && q >= split;
+        const int sh = second ? shift : 0;
+        const int32_t a = sk[q + sh];
+        const uint32_t me = gene_of(gene, genes, si[q + sh]);
+        const float v = __int_as_float(a ^ ((a >> 31) & 0x7FFFFFFF));
+        const int b = bucket(v, nbs) + (second ? nbs : 0);
+        const int hi = (int)cnt[b], lo = b > 0 ? (int)cnt[b - 1] : 0;
+        int r = lo;
+        for (int k = lo; k < hi; ++k) {
+            const int32_t x = sk[k + sh];
+            r += (x < a || (x == a && gene_of(gene, genes, si[k + sh]) < me)) ? 1 : 0;
         }
-        perm[out0 + r] = x;
+        rank[j] = (uint16_t)r;
     }
+    g.sync();
+#pragma unroll 1
+    for (int q = tid, j = 0; q < n; q += T, ++j) perm[rank[j]] = si[q + (SPLIT && q >= split ? shift : 0)];
 }
 
 // equal keys in a thread's window: the window took them in position order; by index instead
@@ -292,8 +307,7 @@ __device__ __forceinline__ void sort_row(int n, int split, const RowBuf& s, cons
             if (SPLIT) sort_heavy_segment<T>(s.sk + seg1, s.si + seg1, n - split, t, g.rg, gene, genes);
             for (int p = t; p < n; p += T) s.perm[p] = s.si[p < gap0 ? p : p + shift];
         } else {
-            rank_loop<T>(s.sk, s.si, s.perm, 0, gap0, 0, w, t, gene, genes);
-            if (SPLIT) rank_loop<T>(s.sk, s.si, s.perm, seg1, n - split, split, w, t, gene, genes);
+            rank_buckets<T, SPLIT>(s.sk, s.si, s.cnt, s.perm, n, split, shift, s.nb, bucket, t, g.rg, gene, genes);
         }
         g.sync();
         return;
