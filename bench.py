@@ -10,7 +10,7 @@ tour length kernel + elite-partition sort) of the device-resident solver.
 N > 1 runs N independent replicas (one instance per GPU, no collective: islands and
 instances are independent units), launched one process per GPU by torch.distributed.run.
 One timed step is a stretch of GENS_PER_STEP generations of the device-resident solver
-(one evolve call: captured CUDA graphs of 16 generations each), with L2 flushed (a 256 MiB
+(one evolve call: cooperative launches of up to 128 generations), with L2 flushed (a 256 MiB
 write) before every step, outside its CUDA-event bracket; inside a step the 16 MB
 population stays L2-resident as it does in a solver run.  The JSON line's `value` is
 whole-job generations per second with the population resident in HBM;
@@ -346,7 +346,7 @@ def run_ours(args, rank, world):
             "e2e": e2e,
             "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
                          "frac": achieved / peak, "traffic": profile_traffic(),
-                         "kernel": "bk::row_kernel<256,1> (fused crossover/mutant/decode/tour length), "
+                         "kernel": "bk::row_kernel<64,0> (fused crossover/mutant/decode/tour length), "
                                    "timed through brkga_generation_step",
                          "traffic_note": "DRAM bytes per launch from profiles/row_kernel_tsp_n1000_p2048.md",
                          "engine_tile": {"threads": s_info[0], "groups": s_info[1], "grid": s_info[2],
@@ -358,7 +358,8 @@ def run_ours(args, rank, world):
                          # kernel's elapsed time)
                          "smem": {"wavefront_pct_of_peak": profile_figure("smem_wavefront_pct_of_peak"),
                                   "source": "profiles/row_kernel_tsp_n1000_p2048.md"}},
-            "gpu_launches": 2 * args.steps * gps,
+            # one population evolves up to 128 generations a launch
+            "gpu_launches": args.steps * -(-gps // 128),
             # rows decoded and evaluated per generation: children and mutants (elites keep
             # their fitness, as the reference's host path does)
             "individual_evaluations_per_s": value * (POP - ELITE),
