@@ -64,3 +64,15 @@ def test_every_tile_same_run(cuda, threads, monkeypatch):
     np.testing.assert_array_equal(keys, rk)
     np.testing.assert_array_equal(fit, rf)
     s.close()
+
+
+@pytest.mark.parametrize("crowd", [9, 10, 20, 31, 32, 33])
+@pytest.mark.parametrize("n", [40, 129, 700])
+def test_crowded_buckets_of_shifted_keys(cuda, n, crowd):
+    """MO-VRP sorts by shifted keys through a bucket map of its own"""
+    xy, dem, cap, V = I.movrp_instance(n, seed=n)
+    po = O.OracleProblem(O.MOVRP, n, xy=xy, w=dem, machines=V, vcap=cap)
+    keys = crowded_keys(n, crowd, seed=n + crowd)[:-1]
+    obj, perm = eval_gpu(B().movrp(xy, dem, cap, V), keys, cuda)
+    np.testing.assert_array_equal(perm, O.decode_problem(po, keys))
+    np.testing.assert_array_equal(obj.view(np.uint32), O.evaluate(po, keys).view(np.uint32))
