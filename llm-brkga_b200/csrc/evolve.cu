@@ -14,10 +14,11 @@
 //   swords[rank]           row of that rank and the step
 // A CTA waits for the words it reads: all fitness words before it ranks its own rows, the
 // two parents' (or one elite's) rank words before it builds a row.  The fitness words order
-// all else: a row's keys and fitness are written before its word (release), and every CTA
-// has seen every word of the step (acquire) before it reads any row of it; a buffer is
-// overwritten two steps later, when every CTA has passed the step between.  The rank words
-// carry nothing but their value.
+// all else: a row's keys and fitness are written before its word (the group's threads meet,
+// then one of them releases the word), and every CTA has seen every word of the step (acquire)
+// before it reads any row of it; a buffer is overwritten two steps later, when every CTA has
+// passed the step between.  The rank words carry nothing but their value: whoever reads one
+// has ranked the step it belongs to, and so has acquired all of that step's rows.
 //
 // Results are those of the row and rank kernels: the same row code, the same order by
 // (fitness, row).

@@ -58,8 +58,9 @@ __device__ __forceinline__ int row_of_task(const PopDesc& sd, int task) {
 }
 
 // Row r of population sd (MODE_LSEARCH: the r-th best row).  from: the rows it is built from
-// (parents, the elite row copied, the searched row) where the caller has resolved them; pts: the instance data staged in shared
-// memory, or null.
+// (parents, the elite row copied, the searched row) where the caller has resolved them; pts:
+// the instance data staged in shared memory, or null.  Where a row was written, the group's threads have met (g.sync) when this
+// returns: any one of them may then publish the row for all.
 template <int T, int CLS, bool COH>
 __device__ __forceinline__ void row_work(const RowLaunch& L, const PopDesc& sd, int mode, int r, const int2* from,
                                          float* pts, const RowBuf& s, const RowGroup<T>& g) {
@@ -158,6 +159,7 @@ __device__ __forceinline__ void row_work(const RowLaunch& L, const PopDesc& sd, 
         float4* o = reinterpret_cast<float4*>(dst + (size_t)r * ld);
         for (int q = t; q < ld / 4; q += T) o[q] = row_ld<COH>(a + q);
         if (t < m) sd.fit[fbuf][(size_t)r * m + t] = row_ld<COH>(sd.fit[cur] + (size_t)sr * m + t);
+        g.sync();
         return;
     }
 
