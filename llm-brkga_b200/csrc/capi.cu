@@ -287,8 +287,12 @@ void tune_store(int kind, int n, int rows, const RowTile& t) {
 }
 
 int32_t tile_setup(const RowTile& t, int kind, int n, int pts, int rows, TunedTile* out) {
+    // a forced tile, or one from a cache file: anything may stand there
+    if (!tile_covers(t.block, n))
+        return fail(BRKGA_ERR_UNSUPPORTED, "no row kernel with " + std::to_string(t.block) + " threads covers " +
+                                               std::to_string(n) + " keys");
     TunedTile tt;
-    tt.tile = t;
+    tt.tile = RowTile{t.block, tile_groups(t.block, n)};
     tt.stage = stage_fits(t, n, pts, kind);
     tt.groups_per_cta = row_groups_per_cta(t, n, pts, kind, tt.stage, rows);
     const size_t smem = row_smem_bytes(t, n, pts, kind, tt.stage, tt.groups_per_cta);

@@ -34,7 +34,10 @@ struct Task {
     int32_t row;
 };
 
-// tile shape chosen per size bucket: threads per row and float4 groups per thread
+// tile shape chosen per size bucket: threads per row and float4 groups per thread.  A thread
+// holds the ranks of its keys in an array of this many groups (row_group.cuh), so no row is
+// launched with fewer threads than that covers.
+constexpr int kMaxTileGroups = 16;
 struct RowTile {
     int block;
     int groups;
@@ -82,6 +85,8 @@ int row_max_n_global();
 bool row_needs_global(int n, int pts, int kind);
 size_t row_global_stride(int max_n);
 int row_global_grid(int rows, int max_n);
+// whether a compiled kernel has this many threads a row and they cover n keys
+bool tile_covers(int block, int n);
 // one-time set-up for a tile / shared-memory size: raises the dynamic shared-memory limit
 // and returns the resident CTAs per SM (0 if the tile cannot run with that much memory)
 cudaError_t prepare_rows(const RowTile& tile, int kind, int groups_per_cta, size_t smem, int* per_sm);

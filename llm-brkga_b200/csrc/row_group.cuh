@@ -144,8 +144,6 @@ __device__ __noinline__ void sort_heavy_segment(int32_t* k, uint16_t* x, int n, 
 // neighbours as that bucket holds, a generation of a converged population (n = 1000, P = 2048)
 // took 48.8 us, now 27.5 (rows that fit the window: 17.7).  cnt holds the buckets' ends and is
 // overwritten by the permutation, so the ranks wait in local memory.
-constexpr int kMaxGroups = 16;  // a thread's keys at most, by four
-
 template <int T, bool SPLIT, typename BucketF>
 __device__ __noinline__ void rank_buckets(const int32_t* sk, const uint16_t* si, const uint32_t* cnt, uint16_t* perm, int n,
                                           int split, int shift, int nb, BucketF bucket, int tid, int rg,
@@ -154,7 +152,7 @@ __device__ __noinline__ void rank_buckets(const int32_t* sk, const uint16_t* si,
     g.tid = tid;
     g.rg = rg;
     const int nbs = SPLIT ? nb / 2 : nb;
-    uint16_t rank[4 * kMaxGroups];
+    uint16_t rank[4 * kMaxTileGroups];  // tile_covers: n <= T * 4 * kMaxTileGroups
 #pragma unroll 1
     for (int q = tid, j = 0; q < n; q += T, ++j) {
         const bool second = SPLIT && q >= split;

@@ -142,12 +142,21 @@ __global__ void __launch_bounds__(T * max_groups(T), 1) row_kernel(RowLaunch L) 
 
 int tile_groups(int block, int n) { return (n + 4 * block - 1) / (4 * block); }
 
-// every thread count that gives a thread 1 .. 16 groups of four keys, fewest threads first
+bool tile_covers(int block, int n) {
+    bool compiled = false;
+#define X(B) compiled = compiled || block == B;
+    BK_TILES(X)
+#undef X
+    return compiled && tile_groups(block, n) <= kMaxTileGroups;
+}
+
+// every thread count that gives a thread 1 .. kMaxTileGroups groups of four keys, fewest threads
+// first
 int tile_candidates(int n, RowTile* out, int cap) {
     int c = 0;
     for (int b = 32; b <= 1024; b *= 2) {
         const int g = tile_groups(b, n);
-        if (g > 16 || c >= cap) continue;
+        if (!tile_covers(b, n) || c >= cap) continue;
         out[c++] = RowTile{b, g};
         if (g == 1) break;
     }
@@ -159,7 +168,7 @@ int tile_candidates(int n, RowTile* out, int cap) {
 // generation's rows with 32 threads, 21 with 64, 36 with 128)
 RowTile pick_tile(int n, int kind) {
     if (n > row_max_n()) return RowTile{0, 0};
-    if ((kind == JOBSCHED || kind == CONTINUOUS) && tile_groups(32, n) <= 16) return RowTile{32, tile_groups(32, n)};
+    if ((kind == JOBSCHED || kind == CONTINUOUS) && tile_covers(32, n)) return RowTile{32, tile_groups(32, n)};
     for (int b = 32; b < 1024; b *= 2)
         if (tile_groups(b, n) <= 4) return RowTile{b, tile_groups(b, n)};
     return RowTile{1024, tile_groups(1024, n)};
@@ -255,7 +264,7 @@ cudaError_t prepare_rows(const RowTile& tile, int kind, int groups_per_cta, size
 cudaError_t launch_rows(const RowLaunch& L, int kind, const RowTile& tile, int grid, cudaStream_t s) {
     if (tile.block == 0) return launch_rows_global(L, kind, grid, s);
     RowFn fn = row_fn(tile, row_class(kind));
-    if (!fn) return cudaErrorInvalidValue;
+    if (!fn || !tile_covers(tile.block, L.max_n)) return cudaErrorInvalidValue;
     if (L.ntasks <= 0 || grid <= 0) return cudaSuccess;
     const int groups = L.groups_per_cta < 1 ? 1 : L.groups_per_cta;
     const int unit = L.tasks ? (L.task_group < 1 ? 1 : L.task_group) : groups;
