@@ -212,6 +212,12 @@ void fill_instance(PopDesc& d, const ProblemData& pd) {
     d.lo = pd.lo;
     d.hi = pd.hi;
     d.maximize = pd.maximize;
+    d.wait_polls = wait_polls();
+}
+
+uint32_t wait_polls() {
+    const char* v = std::getenv("BRKGA_WAIT_POLLS");
+    return v && *v ? (uint32_t)std::min<unsigned long>(std::strtoul(v, nullptr, 10), kWaitPolls) : kWaitPolls;
 }
 
 int points_of(const ProblemData& pd) {

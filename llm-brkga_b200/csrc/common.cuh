@@ -155,8 +155,12 @@ struct PopDesc {
     // TSPJ random 2-opt local search period (0 = off)
     int32_t ls_interval;
     int32_t stuck;            // a bounded wait between a launch's CTAs ran out
+    uint32_t wait_polls;      // polls of one such wait (kWaitPolls unless BRKGA_WAIT_POLLS says otherwise)
     int32_t* stuck_host;      // pinned copy of it for a call that reads no descriptor back, or null
 };
+
+// polls of one wait for another CTA of the same launch: about a second, a step is microseconds
+constexpr uint32_t kWaitPolls = 1u << 22;
 
 __host__ __device__ __forceinline__ bool at_limit(const PopDesc& d) { return d.gen_limit != 0u && d.gen >= d.gen_limit; }
 

@@ -83,6 +83,9 @@ void fill_instance(PopDesc& d, const ProblemData& pd);
 int points_of(const ProblemData& pd);
 bool stage_fits(const RowTile& t, int n, int pts, int kind);
 uint32_t prob_threshold(double p);
+// polls of a wait between the CTAs of one launch: BRKGA_WAIT_POLLS when set (a small number makes
+// the waits run out, for tests of what follows), else kWaitPolls
+uint32_t wait_polls();
 
 // Tile autotuner: times every candidate tile (capacity covering n) on `launch`, which
 // must enqueue one representative row-kernel launch for the tile and grid it is given on

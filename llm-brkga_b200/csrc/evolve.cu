@@ -39,16 +39,14 @@ struct EvolveArgs {
     int gens, ls_count;
 };
 
-constexpr uint32_t kSpinLimit = 1u << 22;  // polls of one wait: about a second; a step is microseconds
-
 __device__ __forceinline__ unsigned long long word_of(uint32_t step, uint32_t v) {
     return ((unsigned long long)step << 32) | v;
 }
 
 // the word's value once it carries `step`; 0 and *stuck set when the wait runs out
-__device__ __forceinline__ uint32_t await(const unsigned long long* p, uint32_t step, int* stuck) {
+__device__ __forceinline__ uint32_t await(const unsigned long long* p, uint32_t step, uint32_t polls, int* stuck) {
     unsigned long long w;
-    for (uint32_t n = 0; n < kSpinLimit; ++n) {
+    for (uint32_t n = 0; n < polls; ++n) {
         asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(w) : "l"(p) : "memory");
         if ((uint32_t)(w >> 32) == step) return (uint32_t)w;
         if ((n & 255u) == 255u && *static_cast<volatile int*>(stuck)) break;  // the CTA has given up
@@ -105,7 +103,7 @@ __global__ void __launch_bounds__(T * max_groups(T), 1) evolve_kernel(EvolveArgs
     auto rank_rows = [&](uint32_t step) {
         const unsigned long long* w = A.fwords + (size_t)(step & 1u) * P;
         for (int j = threadIdx.x; j < round_up(P, 4); j += blockDim.x)
-            okeys[j] = (j < P) ? await(w + j, step, &stuck) : 0xFFFFFFFFu;
+            okeys[j] = (j < P) ? await(w + j, step, sd.wait_polls, &stuck) : 0xFFFFFFFFu;
         asm volatile("fence.acq_rel.gpu;" ::: "memory");
         __syncthreads();
         for (int q = warp; c0 + grid * q < P; q += warps) {
@@ -142,7 +140,7 @@ __global__ void __launch_bounds__(T * max_groups(T), 1) evolve_kernel(EvolveArgs
                 if (ranked == 0) {
                     from = make_int2(sd.sorted[pk.x], sd.sorted[pk.y]);
                 } else if (T == 32 || g.tid < 32) {
-                    from.x = (int)await(A.swords + ((lane & 1) ? pk.y : pk.x), ranked, &stuck);
+                    from.x = (int)await(A.swords + ((lane & 1) ? pk.y : pk.x), ranked, sd.wait_polls, &stuck);
                     from.y = __shfl_sync(0xffffffffu, from.x, 1);
                     from.x = __shfl_sync(0xffffffffu, from.x, 0);
                 }

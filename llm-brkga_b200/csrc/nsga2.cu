@@ -749,6 +749,9 @@ __device__ __forceinline__ bool select_active(const PopDesc& d, int mode) {
 //    barrier took 1900 and one warp's stores and a cluster barrier 1300.  Four masks go round:
 //    a CTA sends mask k + 3 only after every other CTA has sent mask k + 2, and none does
 //    before it is done reading masks k - 1 and k.
+//  - Waits are bounded.  A CTA whose wait runs out gives up, but words may still be on their way
+//    to it: it says how many masks it has sent, sends the one that others wait for, and leaves
+//    when every mask that was sent has arrived (a second bounded wait).
 //  - A step (four points) is counted only if one of its points can come to zero: its count less
 //    the points that joined since it was last counted.  About half the steps of a front are.
 //  - Counts are bound by logic (two cycles a warp) and population counts (eight): 16 words take
@@ -794,8 +797,6 @@ __device__ __forceinline__ int count_bits(const uint32_t (&x)[n]) {
 
 __device__ __forceinline__ uint32_t shared_addr(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
 
-constexpr uint32_t kMaskPolls = 1u << 24;  // polls of one wait: most of a second; a front is microseconds
-
 template <int WL>
 __global__ void __launch_bounds__(kPeelThreads, 1) nsga_peel_rows_kernel(PopDesc* dd, int mode) {
     dep_wait();
@@ -804,12 +805,14 @@ __global__ void __launch_bounds__(kPeelThreads, 1) nsga_peel_rows_kernel(PopDesc
     __shared__ __align__(16) uint32_t F[4][NW];  // the points of the fronts 0..k in F[k & 3]
     __shared__ __align__(16) uint16_t out[kPeelThreads / 32];  // the CTA's part of the next mask
     __shared__ __align__(8) uint64_t bar[4];  // of each mask: every CTA's part has arrived
+    __shared__ int gave_up[16];  // the last mask that each CTA of the cluster sent before it gave up, or -1
     cg::cluster_group cluster = cg::this_cluster();
     const int csize = (int)cluster.num_blocks(), crank = (int)cluster.block_rank();
     PopDesc& d = dd[blockIdx.x / csize];
     if (!select_active(d, mode)) return;  // the same decision in every CTA of the cluster
     const int N = (mode == 0) ? 2 * d.P : d.P;
     const int Wmax = d.domW;
+    const uint32_t polls = 4u * d.wait_polls;  // a poll of shared memory is shorter than one of L2
     const int t = threadIdx.x, lane = t & 31, warp = t >> 5, sub = lane & 7;
     // A CTA has pairs of words (64 points each) from the four quarters of the points: a pool's
     // survivors come in the order of their last fronts, so neighbours are at work together.
@@ -821,6 +824,7 @@ __global__ void __launch_bounds__(kPeelThreads, 1) nsga_peel_rows_kernel(PopDesc
         asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(shared_addr(&bar[t])) : "memory");
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
+    if (t < 16) gave_up[t] = -1;
     // (Words past N stay zero in the masks: rows may hold anything there.)
     for (int w = t; w < NW; w += kPeelThreads) {
         F[1][w] = (w < N / 32) ? 0xFFFFFFFFu : (w == N / 32 && (N & 31)) ? (1u << (N & 31)) - 1u : 0u;
@@ -865,6 +869,22 @@ __global__ void __launch_bounds__(kPeelThreads, 1) nsga_peel_rows_kernel(PopDesc
         cnt[2] = (int)(pk[1] & 0xFFFFu), cnt[3] = (int)(pk[1] >> 16);
     };
     uint32_t ranked = 0u, mine = 0u;  // the warp's points in the fronts so far, in the next one: bit 4 s + lane / 8
+    // the CTA's part of mask b to every CTA, one pair of words a thread
+    auto deliver = [&](int b) {
+        if (t < 4 * csize) {
+            const int q = t & 3;
+            const uint32_t to = shared_addr(&F[b][word_of(q)]), at = shared_addr(&bar[b]);
+            if (t == 0)
+                asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(at), "r"(32 * csize) : "memory");
+            const uint2 v = reinterpret_cast<const uint2*>(out)[q];
+            uint32_t rto, rat;
+            asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(rto) : "r"(to), "r"(t >> 2));
+            asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(rat) : "r"(at), "r"(t >> 2));
+            asm volatile("st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.v2.b32 [%0], {%1, %2}, [%3];"
+                         ::"r"(rto), "r"(v.x), "r"(v.y), "r"(rat)
+                         : "memory");
+        }
+    };
     // points of the steps `act` at or below zero and not ranked yet join the next front: the
     // CTA's 256 bits of mask b gathered, then sent to every CTA
     auto send_front = [&](int b, uint32_t act, const int (&left)[4]) {
@@ -881,25 +901,13 @@ __global__ void __launch_bounds__(kPeelThreads, 1) nsga_peel_rows_kernel(PopDesc
         ranked |= mine;
         if (lane == 0) out[warp] = (uint16_t)ranked;
         __syncthreads();
-        if (t < 4 * csize) {  // one pair of words to one CTA
-            const int q = t & 3;
-            const uint32_t to = shared_addr(&F[b][word_of(q)]), at = shared_addr(&bar[b]);
-            if (t == 0)
-                asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(at), "r"(32 * csize) : "memory");
-            const uint2 v = reinterpret_cast<const uint2*>(out)[q];
-            uint32_t rto, rat;
-            asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(rto) : "r"(to), "r"(t >> 2));
-            asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(rat) : "r"(at), "r"(t >> 2));
-            asm volatile("st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.v2.b32 [%0], {%1, %2}, [%3];"
-                         ::"r"(rto), "r"(v.x), "r"(v.y), "r"(rat)
-                         : "memory");
-        }
+        deliver(b);
     };
-    // front k's mask is complete; false (in every thread of the CTA) when a wait ran out
-    auto await_front = [&](int k) {
+    // mask k is complete; false (in every thread of the CTA) when the wait ran out
+    auto await_front = [&](int k, uint32_t polls) {
         const uint32_t at = shared_addr(&bar[k & 3]), parity = (uint32_t)(k >> 2) & 1u;
         uint32_t done = 0u;
-        for (uint32_t n = 0; n < kMaskPolls && !done; ++n)
+        for (uint32_t n = 0; n < polls && !done; ++n)
             asm volatile(
                 "{.reg .pred p;\n\t"
                 "mbarrier.test_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\t"
@@ -920,10 +928,11 @@ __global__ void __launch_bounds__(kPeelThreads, 1) nsga_peel_rows_kernel(PopDesc
     // thread 0 of the cluster's first CTA records the front table (start of each front in
     // rank order, the cut front) for the grid-wide crowding and placement of mode 0
     int32_t* const ft = (crank == 0 && t == 0) ? d.nft : nullptr;
+    int k = 0;
     bool stuck = false;
-    for (int k = 0;; ++k) {
+    for (;; ++k) {
         const uint32_t* const f = F[k & 3];
-        if (!await_front(k)) {
+        if (!await_front(k, polls)) {
             stuck = true;
             break;
         }
@@ -992,16 +1001,28 @@ __global__ void __launch_bounds__(kPeelThreads, 1) nsga_peel_rows_kernel(PopDesc
             break;
         }
     }
+    if (stuck) {
+        if (t < csize) *cluster.map_shared_rank(&gave_up[crank], t) = k;
+        if (t == 0) {
+            d.stuck = 1;
+            if (d.stuck_host) *d.stuck_host = 1;
+        }
+    }
     __syncwarp();
     asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
-    if (stuck && t == 0) {
-        d.stuck = 1;
-        if (d.stuck_host) *d.stuck_host = 1;
-    }
     if (lane < 16 && p0 + lane < N && !((ranked >> lane) & 1u)) d.domcnt[p0 + lane] = rest;
     // no CTA leaves while another may still send to it
     __syncwarp();
     asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+    if (stuck) {
+        // Every CTA has sent all that it is going to.  A CTA that sent mask k + 1 waits for it, so
+        // it gave up too, and none got further without this CTA's part.  (CTAs that did not give
+        // up have all of mask k, the last one sent then.)
+        int last = k;
+        for (int c = 0; c < csize; ++c) last = max(last, gave_up[c]);
+        if (last > k) deliver(last & 3);
+        for (int b = k; b <= last; ++b) await_front(b, 4u * kWaitPolls);
+    }
 }
 
 using PeelFn = void (*)(PopDesc*, int);
@@ -1932,6 +1953,7 @@ int32_t brkga_pareto_rank_bitmatrix(const float* d_obj, int32_t N, int32_t m, in
         hd.domW = W;
         hd.domcnt = d_rank;
         hd.stuck_host = g_op_stuck;
+        hd.wait_polls = wait_polls();
         PopDesc* dd = reinterpret_cast<PopDesc*>((char*)buf + doff);
         if ((e = cudaMemcpyAsync(dd, &hd, sizeof(hd), cudaMemcpyHostToDevice, st)) != cudaSuccess)
             return cuda_fail(e, "peel descriptor");
