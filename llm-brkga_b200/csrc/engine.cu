@@ -240,6 +240,16 @@ static int32_t sync_descs_to_host(brkga_engine* e) {
     return BRKGA_OK;
 }
 
+// host descriptors of a population about to be built anew
+static void reset_descs(brkga_engine* e) {
+    for (PopDesc& d : e->hd) {
+        d.cur = 0;
+        d.gen = 0;
+        d.stuck = 0;
+        d.wait_polls = wait_polls();
+    }
+}
+
 static int32_t grow_history(brkga_engine* e, int need) {
     Population& p = e->pop;
     if (need <= p.hist_cap) return BRKGA_OK;
@@ -497,11 +507,7 @@ int32_t brkga_initialize(brkga_engine* e) {
     }
     const Shape& sh = e->pop.sh;
     // reset generation counters / buffer index on the device
-    for (auto& d : e->hd) {
-        d.cur = 0;
-        d.gen = 0;
-        d.stuck = 0;
-    }
+    reset_descs(e);
     cudaError_t err = cudaMemcpyAsync(e->dd, e->hd.data(), sizeof(PopDesc) * e->hd.size(),
                                       cudaMemcpyHostToDevice, e->stream);
     if (err != cudaSuccess) return cuda_fail(err, "descriptor upload");
@@ -803,10 +809,7 @@ int32_t brkga_external_begin(brkga_engine* e, int32_t dense, float** d_keys, flo
         // NSGA-II refill rows, built by the commit that reported them
     } else if (!e->initialized) {
         // Population::initialize (core/population.hpp:107-124)
-        for (auto& d : e->hd) {
-            d.cur = 0;
-            d.gen = 0;
-        }
+        reset_descs(e);
         err = cudaMemcpyAsync(e->dd, e->hd.data(), sizeof(PopDesc) * e->hd.size(), cudaMemcpyHostToDevice, e->stream);
         if (err == cudaSuccess) {
             if (sh.mo) {

@@ -84,6 +84,7 @@ __global__ void __launch_bounds__(T * max_groups(T), 1) evolve_kernel(EvolveArgs
         reinterpret_cast<uint32_t*>(&sd)[i] = reinterpret_cast<const uint32_t*>(A.desc)[i];
     zero_counters<T>(s, g.tid);
     __syncthreads();
+    if (sd.stuck) return;  // an earlier launch gave up a wait
     const bool staged = L.stage_xy && has_points(sd.kind);
     if (staged) stage_points<CLS>(sd, pts);
     const int P = sd.P, E = sd.E, M = sd.M, mx = sd.maximize;

@@ -730,8 +730,10 @@ __device__ float block_min_f(float v, float* red) {
 
 // Selection launches (core/population.hpp:409-517): mode 0 works on the 2P pool of fit[cur]
 // and picks the survivors; mode 1 ranks the P population (initialisation); mode 2 does
-// the same only for populations the diversity pass rebuilt (*nu < P).
+// the same only for populations the diversity pass rebuilt (*nu < P).  A population whose peel
+// gave up a wait has a front table that is half written: nothing of it is selected any more.
 __device__ __forceinline__ bool select_active(const PopDesc& d, int mode) {
+    if (d.stuck) return false;
     if (mode == 0) return !at_limit(d);
     if (mode == 2) return d.advanced && __ldg(d.nu) < d.P;
     return true;
@@ -1285,7 +1287,7 @@ __global__ void __launch_bounds__(kFrontWarps * 32) nsga_cut_kernel(PopDesc* dd)
     extern __shared__ unsigned long long ckeys[];  // [cut front size]
     __shared__ uint32_t s_min;
     PopDesc& d = dd[blockIdx.y];
-    if (at_limit(d)) {
+    if (!select_active(d, 0)) {
         if (blockIdx.x == 0 && threadIdx.x == 0) d.advanced = 0;
         return;
     }

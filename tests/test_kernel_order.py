@@ -43,3 +43,17 @@ def test_words_follow_row_work():
     for at in releases:
         loop = kernel[kernel.rindex("for (int q = g.rg", 0, at):at]
         assert "row_work<" in loop and "if (g.tid == 0)" in loop[loop.index("row_work<"):]
+
+
+def test_selection_stops_at_a_wait_that_ran_out():
+    """a peel that gave up leaves a half-written front table: the kernels that place survivors by
+    it start with the check"""
+    text = source("nsga2.cu")
+    assert "if (d.stuck) return false;" in body(text, "bool select_active(")
+    kernels = ["nsga_peel_rows_kernel(PopDesc", "nsga_front_crowd_kernel(PopDesc", "nsga_cut_kernel(PopDesc",
+               "nsga_order_kernel(PopDesc", "nsga_select_kernel(PopDesc"]
+    for k in kernels:
+        start = body(text, k)
+        assert "select_active(" in start[:start.index("return;")], k
+    kernel = body(source("evolve.cu"), "evolve_kernel(EvolveArgs A)")
+    assert kernel.index("if (sd.stuck) return;") < kernel.index("stage_points")
