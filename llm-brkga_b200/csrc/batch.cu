@@ -67,13 +67,15 @@ struct Group {
     // balanced, 8 there cost 8%)
     int task_group = 1;
     int32_t* work = nullptr;  // the row kernel's dynamic dealing counter (launches on `stream`)
+    int32_t* flag = nullptr;  // set when a wait of a member's launches ran out
 };
 
 // the group's stream and its zeroed row-dealing counter
 static int32_t group_start(Group& g) {
     cudaError_t e = cudaStreamCreateWithFlags(&g.stream, cudaStreamNonBlocking);
     if (e != cudaSuccess) return cuda_fail(e, "stream");
-    int32_t st = dev_alloc((void**)&g.work, 8, g.stream);
+    int32_t st = flag_take(&g.flag);
+    if (st == BRKGA_OK) st = dev_alloc((void**)&g.work, 8, g.stream);
     if (st != BRKGA_OK) return st;
     if ((e = cudaMemsetAsync(g.work, 0, 8, g.stream)) != cudaSuccess) return cuda_fail(e, "work counter");
     return BRKGA_OK;
@@ -84,6 +86,8 @@ static void group_stop(Group& g) {
     if (g.work) dev_free(g.work, g.stream);
     g.work = nullptr;
     cudaStreamSynchronize(g.stream);
+    flag_give(g.flag);
+    g.flag = nullptr;
     cudaStreamDestroy(g.stream);
     g.stream = nullptr;
 }
@@ -201,7 +205,10 @@ static int32_t build_plan(Group& g) {
         m->first = (int)g.hd.size();
         m->ndesc = m->sh.k;
         for (int i = 0; i < m->sh.k; ++i) g.hd.push_back(m->pop.hd_template[i]);
-        for (int i = 0; i < m->sh.k; ++i) g.hd[m->first + i].gen_limit = m->limit;
+        for (int i = 0; i < m->sh.k; ++i) {
+            g.hd[m->first + i].gen_limit = m->limit;
+            g.hd[m->first + i].stuck_host = g.flag;
+        }
         if (m->sh.mo) {
             ++g.nn;
             g.maxP_n = std::max(g.maxP_n, m->sh.Pi);
@@ -254,11 +261,20 @@ static int32_t pull_state(Group& g) {
     cudaError_t e = cudaStreamSynchronize(g.stream);
     if (e == cudaSuccess) e = cudaMemcpy(g.hd.data(), g.dd, sizeof(PopDesc) * nd, cudaMemcpyDeviceToHost);
     if (e != cudaSuccess) return cuda_fail(e, "descriptor read-back");
-    for (const PopDesc& d : g.hd)
-        if (d.stuck) return fail(BRKGA_ERR_TIMEOUT, "a wait between the launch's CTAs ran out; the populations are not valid");
     for (Member* m : g.members)
         for (int i = 0; i < m->ndesc; ++i) m->pop.hd_template[i] = g.hd[m->first + i];
     return BRKGA_OK;
+}
+
+// a wait of one of the member's launches ran out (host descriptors current)
+static bool gave_up(const Group& g, const Member* m) {
+    for (int i = 0; i < m->ndesc; ++i)
+        if (g.hd[m->first + i].stuck) return true;
+    return false;
+}
+
+static int32_t wait_failed() {
+    return fail(BRKGA_ERR_TIMEOUT, "a wait between a launch's CTAs ran out; the batch's populations are not valid");
 }
 
 static cudaError_t enqueue_generation(Group& g, bool mig) {
@@ -624,6 +640,7 @@ int32_t brkga_batch_evolve(brkga_batch* b, int32_t generations) {
     for (Member* m : b->g.members)
         if ((int)b->gen + generations + 1 > m->pop.hist_cap)
             return fail(BRKGA_ERR_INVALID, "batch evolved past a member's max_generations");
+    if (flag_set(b->g.flag)) return wait_failed();
     NvtxRange range("batch generations", b->gen + 1u, b->gen + (unsigned)generations);
     cudaError_t e = run_generations(b->g, b->gen, generations, true);
     if (e != cudaSuccess) return cuda_fail(e, "batch evolve");
@@ -636,7 +653,7 @@ int32_t brkga_batch_synchronize(brkga_batch* b) {
     DeviceGuard guard(b->g.device);
     cudaError_t e = cudaStreamSynchronize(b->g.stream);
     if (e != cudaSuccess) return cuda_fail(e, "batch stream");
-    return BRKGA_OK;
+    return flag_set(b->g.flag) ? wait_failed() : BRKGA_OK;
 }
 
 int32_t brkga_batch_get_best(brkga_batch* b, float* best) {
@@ -645,6 +662,7 @@ int32_t brkga_batch_get_best(brkga_batch* b, float* best) {
     DeviceGuard guard(b->g.device);
     int32_t st = pull_state(b->g);
     if (st != BRKGA_OK) return st;
+    if (flag_set(b->g.flag)) return wait_failed();
     std::vector<Leader> lead;
     if ((st = read_leaders(b->g, 0, (int)b->g.hd.size(), lead)) != BRKGA_OK) return st;
     // members are stored single-objective first; report in creation order
@@ -664,6 +682,7 @@ int32_t brkga_batch_get_best_keys(brkga_batch* b, int32_t index, float* keys, fl
     DeviceGuard guard(b->g.device);
     int32_t st = pull_state(b->g);
     if (st != BRKGA_OK) return st;
+    if (flag_set(b->g.flag)) return wait_failed();
     Member* m = nullptr;
     for (Member* x : b->g.members)
         if (x->prm_index == index) m = x;
@@ -797,7 +816,7 @@ static void server_retire(brkga_server* s, Request* r, int state) {
     if (r->m) {
         std::vector<Leader> lead;
         float v[2];
-        if (read_leaders(s->g, r->m->first, r->m->ndesc, lead) == BRKGA_OK &&
+        if (state != REQ_FAILED && read_leaders(s->g, r->m->first, r->m->ndesc, lead) == BRKGA_OK &&
             member_best(s->g, r->m, lead.data(), v) == BRKGA_OK) {
             r->best[0] = v[0];
             r->best[1] = v[1];
@@ -932,6 +951,12 @@ int32_t brkga_server_step(brkga_server* s) {
         if ((st = pull_state(g)) != BRKGA_OK) return st;
         for (Request* r : s->active) {
             Member* m = r->m;
+            if (gave_up(g, m)) {  // the other requests go on
+                r->err = BRKGA_ERR_TIMEOUT;
+                server_retire(s, r, REQ_FAILED);
+                changed = true;
+                continue;
+            }
             const bool mx = m->pd->maximize != 0;
             float b = hb[m->first];
             for (int i = 1; i < m->ndesc; ++i) b = mx ? std::max(b, hb[m->first + i]) : std::min(b, hb[m->first + i]);

@@ -156,11 +156,17 @@ struct PopDesc {
     int32_t ls_interval;
     int32_t stuck;            // a bounded wait between a launch's CTAs ran out
     uint32_t wait_polls;      // polls of one such wait (kWaitPolls unless BRKGA_WAIT_POLLS says otherwise)
-    int32_t* stuck_host;      // pinned copy of it for a call that reads no descriptor back, or null
+    int32_t* stuck_host;      // pinned copy of it for calls that read no descriptor back, or null
 };
 
 // polls of one wait for another CTA of the same launch: about a second, a step is microseconds
 constexpr uint32_t kWaitPolls = 1u << 22;
+
+// a launch's wait ran out: the population is left alone until it is initialised again
+__device__ __forceinline__ void set_stuck(PopDesc& d) {
+    d.stuck = 1;
+    if (d.stuck_host) *d.stuck_host = 1;
+}
 
 __host__ __device__ __forceinline__ bool at_limit(const PopDesc& d) { return d.gen_limit != 0u && d.gen >= d.gen_limit; }
 

@@ -143,6 +143,7 @@ struct brkga_engine {
     EvolvePlan evo;            // whole generations in one launch (groups 0: graphs of row and rank launches)
     unsigned long long* evo_words = nullptr;
     uint32_t evo_step = 0;
+    int32_t* flag = nullptr;   // set when a wait of one of its launches ran out
 };
 
 static RowLaunch base_launch(brkga_engine* e, int mode) {
@@ -240,6 +241,15 @@ static int32_t sync_descs_to_host(brkga_engine* e) {
     return BRKGA_OK;
 }
 
+// BRKGA_ERR_TIMEOUT when the population's launches gave up a wait.  The flag only says where to
+// look (it may have been set for a population that has been initialised anew since).
+static int32_t check_waits(brkga_engine* e) {
+    if (!flag_set(e->flag)) return BRKGA_OK;
+    const int32_t st = sync_descs_to_host(e);
+    if (st == BRKGA_OK) *e->flag = 0;
+    return st;
+}
+
 // host descriptors of a population about to be built anew
 static void reset_descs(brkga_engine* e) {
     for (PopDesc& d : e->hd) {
@@ -283,6 +293,7 @@ static void destroy_engine(brkga_engine* e) {
     if (e->gx_special) cudaGraphExecDestroy(e->gx_special);
     nsga_release(e->nsga);
     e->pop.release(e->device);
+    flag_give(e->flag);
     if (e->stream) cudaStreamDestroy(e->stream);
     delete e;
 }
@@ -314,7 +325,7 @@ int32_t brkga_create(brkga_problem* pbh, const brkga_params* params, brkga_engin
         return cuda_fail(err, "stream");
     }
     e->pop.stream = e->stream;
-    if ((st = e->pop.allocate(e->device)) != BRKGA_OK) {
+    if ((st = flag_take(&e->flag)) != BRKGA_OK || (st = e->pop.allocate(e->device)) != BRKGA_OK) {
         destroy_engine(e);
         return st;
     }
@@ -353,6 +364,7 @@ int32_t brkga_create(brkga_problem* pbh, const brkga_params* params, brkga_engin
         d.hist_cap = e->pop.hist_cap;
         d.cur = 0;
         d.gen = 0;
+        d.stuck_host = e->flag;
     }
     // one population: whole generations per launch, where that is the faster way.  The parents of
     // a generation are then drawn by the CTAs that use them
@@ -537,7 +549,8 @@ int32_t brkga_evolve(brkga_engine* e, int32_t generations) {
     }
     std::lock_guard<std::mutex> lk(e->mu);
     DeviceGuard g(e->device);
-    int32_t st = grow_history(e, (int)e->gen + generations + 1);
+    int32_t st = check_waits(e);
+    if (st == BRKGA_OK) st = grow_history(e, (int)e->gen + generations + 1);
     if (st != BRKGA_OK) return st;
     cudaError_t err = cudaSuccess;
     int left = generations;
@@ -591,7 +604,8 @@ int32_t brkga_synchronize(brkga_engine* e) {
     DeviceGuard g(e->device);
     cudaError_t err = cudaStreamSynchronize(e->stream);
     if (err != cudaSuccess) return cuda_fail(err, "engine stream");
-    return BRKGA_OK;
+    std::lock_guard<std::mutex> lk(e->mu);
+    return check_waits(e);
 }
 
 int32_t brkga_run(brkga_engine* e) {
@@ -749,6 +763,8 @@ int32_t brkga_get_fitness_history(brkga_engine* e, float* history, int32_t cap, 
     DeviceGuard g(e->device);
     cudaError_t err = cudaStreamSynchronize(e->stream);
     if (err != cudaSuccess) return cuda_fail(err, "engine stream");
+    const int32_t st = check_waits(e);
+    if (st != BRKGA_OK) return st;
     const Shape& sh = e->pop.sh;
     const int have = std::min<int>((int)e->gen + 1, e->pop.hist_cap);
     const int cnt = std::min(have, (int)cap);

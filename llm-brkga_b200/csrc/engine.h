@@ -25,6 +25,11 @@ int32_t dev_alloc(void** p, size_t bytes, cudaStream_t st);
 void dev_free(void* p, cudaStream_t st);
 size_t pool_reserved(int dev);
 size_t pool_spare(int dev);
+// a pinned word, zero, that kernels set when a wait of theirs runs out (PopDesc::stuck_host); given
+// back when no kernel that has it can be running
+int32_t flag_take(int32_t** out);
+void flag_give(int32_t* f);
+inline bool flag_set(const int32_t* f) { return f && *static_cast<const volatile int32_t*>(f) != 0; }
 int32_t cuda_fail(cudaError_t e, const char* what);
 
 // An NVTX range around a stretch of host work (named like "generations 17-32").  With no

@@ -202,7 +202,7 @@ __global__ void __launch_bounds__(T * max_groups(T), 1) evolve_kernel(EvolveArgs
         A.desc->cur = sd.cur;
         A.desc->gen = sd.gen;
     }
-    if (threadIdx.x == 0 && stuck) A.desc->stuck = 1;
+    if (threadIdx.x == 0 && stuck) set_stuck(*A.desc);
 }
 
 // ---------------------------------------------------------------------------------------

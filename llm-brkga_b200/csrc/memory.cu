@@ -5,6 +5,7 @@
 #include <cstdint>
 #include <map>
 #include <mutex>
+#include <vector>
 
 #include "engine.h"
 
@@ -70,6 +71,54 @@ size_t pool_reserved(int dev) {
     uint64_t v = 0;
     cudaMemPoolGetAttribute(pool, cudaMemPoolAttrReservedMemCurrent, &v);
     return (size_t)v;
+}
+
+// Pinned words that kernels write when a wait between their CTAs runs out, so that a call which
+// waits for its stream anyway sees it without a copy.  Handed out of pages of 1024 (allocating
+// one costs tens of microseconds); a page that is not in use is given back unless it is the last.
+struct FlagPage {
+    int32_t* base;
+    std::vector<int32_t*> spare;
+};
+constexpr int kFlagsPerPage = 1024;
+static std::mutex g_flag_mu;
+static std::vector<FlagPage> g_flag_pages;
+
+int32_t flag_take(int32_t** out) {
+    std::lock_guard<std::mutex> lk(g_flag_mu);
+    FlagPage* from = nullptr;
+    for (FlagPage& p : g_flag_pages)
+        if (!p.spare.empty()) from = &p;
+    if (!from) {
+        FlagPage p{};
+        const cudaError_t e = cudaHostAlloc(&p.base, kFlagsPerPage * sizeof(int32_t), cudaHostAllocPortable | cudaHostAllocMapped);
+        if (e != cudaSuccess) {
+            cudaGetLastError();
+            return fail(BRKGA_ERR_OOM, std::string("pinned flags: ") + cudaGetErrorString(e));
+        }
+        for (int i = kFlagsPerPage; i-- > 0;) p.spare.push_back(p.base + i);
+        g_flag_pages.push_back(std::move(p));
+        from = &g_flag_pages.back();
+    }
+    *out = from->spare.back();
+    from->spare.pop_back();
+    **out = 0;
+    return BRKGA_OK;
+}
+
+void flag_give(int32_t* f) {
+    if (!f) return;
+    std::lock_guard<std::mutex> lk(g_flag_mu);
+    for (size_t i = 0; i < g_flag_pages.size(); ++i) {
+        FlagPage& p = g_flag_pages[i];
+        if (f < p.base || f >= p.base + kFlagsPerPage) continue;
+        p.spare.push_back(f);
+        if ((int)p.spare.size() == kFlagsPerPage && g_flag_pages.size() > 1) {
+            cudaFreeHost(p.base);
+            g_flag_pages.erase(g_flag_pages.begin() + (long)i);
+        }
+        return;
+    }
 }
 
 }  // namespace bk

@@ -1005,10 +1005,7 @@ __global__ void __launch_bounds__(kPeelThreads, 1) nsga_peel_rows_kernel(PopDesc
     }
     if (stuck) {
         if (t < csize) *cluster.map_shared_rank(&gave_up[crank], t) = k;
-        if (t == 0) {
-            d.stuck = 1;
-            if (d.stuck_host) *d.stuck_host = 1;
-        }
+        if (t == 0) set_stuck(d);
     }
     __syncwarp();
     asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
@@ -1875,19 +1872,15 @@ static int32_t static_scratch(uint32_t** out) {
 // scratch of the operator entry points (grow-only, per device)
 static std::mutex g_op_mu;
 static std::map<int, std::pair<void*, size_t>> g_op_buf;
-static int32_t* g_op_stuck = nullptr;  // pinned: a wait in an operator's kernel ran out (read without a copy)
+static int32_t* g_op_stuck = nullptr;  // a wait in an operator's kernel ran out
 
 static int32_t op_scratch(size_t need, void** out) {
     int dev = 0;
     cudaError_t e = cudaGetDevice(&dev);
     if (e != cudaSuccess) return cuda_fail(e, "cudaGetDevice");
     if (!g_op_stuck) {
-        if ((e = cudaHostAlloc(&g_op_stuck, sizeof(int32_t), cudaHostAllocPortable | cudaHostAllocMapped)) != cudaSuccess) {
-            g_op_stuck = nullptr;
-            cudaGetLastError();
-            return fail(BRKGA_ERR_OOM, std::string("operator flag: ") + cudaGetErrorString(e));
-        }
-        *g_op_stuck = 0;
+        const int32_t st = flag_take(&g_op_stuck);
+        if (st != BRKGA_OK) return st;
     }
     auto& b = g_op_buf[dev];
     if (b.second < need) {
@@ -1969,7 +1962,7 @@ int32_t brkga_pareto_rank_bitmatrix(const float* d_obj, int32_t N, int32_t m, in
     }
     // the scratch is shared by later calls: finish before returning
     if ((e = cudaStreamSynchronize(st)) != cudaSuccess) return cuda_fail(e, "peel");
-    if (*static_cast<volatile int32_t*>(g_op_stuck)) {
+    if (flag_set(g_op_stuck)) {
         *g_op_stuck = 0;
         return fail(BRKGA_ERR_TIMEOUT, "a wait between the peel's CTAs ran out; the ranks are not valid");
     }

@@ -91,3 +91,74 @@ def test_one_objective_after_waits_ran_out(cuda, n, P, ls, monkeypatch):
         for a, b in zip(run_population(s, 200), want):
             np.testing.assert_array_equal(a, b)
     s.close()
+
+
+def timeout(call):
+    with pytest.raises(RuntimeError) as e:
+        call()
+    assert e.value.code == TIMEOUT
+
+
+def solvers():
+    import instances as I
+    return {"one": lambda: B().Solver(B().tsp(I.tsp_coords(60, seed=1)), B().params(200, 40, 20, 0.7, 30, seed=5)),
+            "two": lambda: B().Solver(B().bitsp(I.tsp_coords(31, seed=1), I.tsp_coords(31, seed=2)),
+                                      B().params(200, 0, 20, 0.7, 30, seed=5))}
+
+
+@pytest.mark.parametrize("which", ["one", "two"])
+def test_every_call_says_so(cuda, which, monkeypatch):
+    s = solvers()[which]()
+    monkeypatch.setenv("BRKGA_WAIT_POLLS", "0")
+    timeout(s.run)
+    timeout(s.synchronize)
+    timeout(s.get_fitness_history)
+    timeout(s.get_population)
+    timeout(lambda: s.evolve(1))
+    other = solvers()[which]()  # its flag is its own
+    monkeypatch.delenv("BRKGA_WAIT_POLLS")
+    other.run()
+    timeout(s.synchronize)
+    s.run()
+    np.testing.assert_array_equal(s.get_fitness_history(), other.get_fitness_history())
+    s.close()
+    other.close()
+
+
+def test_batch_says_so(cuda, monkeypatch):
+    import instances as I
+    pbs = [B().bitsp(I.tsp_coords(31, seed=1), I.tsp_coords(31, seed=2)), B().tsp(I.tsp_coords(40, seed=3))]
+    prms = [B().params(100, 0, 10, 0.7, 20, seed=1), B().params(100, 20, 10, 0.7, 20, seed=2)]
+    monkeypatch.setenv("BRKGA_WAIT_POLLS", "0")
+    batch = B().Batch(pbs, prms)
+    timeout(batch.synchronize)
+    timeout(lambda: batch.evolve(3))
+    timeout(batch.best)
+    timeout(lambda: batch.best_keys(1))
+    batch.close()
+    monkeypatch.delenv("BRKGA_WAIT_POLLS")
+    batch = B().Batch(pbs, prms)
+    batch.evolve(3)
+    assert np.isfinite(batch.best()[0]).all() and np.isfinite(batch.best()[1, 0])
+    batch.close()
+
+
+def test_server_fails_the_request_alone(cuda, monkeypatch):
+    import instances as I
+    server = B().Server(generations_per_tick=5)
+    monkeypatch.setenv("BRKGA_WAIT_POLLS", "0")
+    bad = server.submit(prm=B().params(100, 0, 10, 0.7, 20, seed=1), kind=B().BITSP_COORDS, n=30,
+                        coords=I.tsp_coords(31, seed=1), coords2=I.tsp_coords(31, seed=2))
+    good = server.submit(prm=B().params(100, 20, 10, 0.7, 20, seed=2), kind=B().TSP_COORDS, n=40,
+                         coords=I.tsp_coords(40, seed=3))
+    server.step()
+    monkeypatch.delenv("BRKGA_WAIT_POLLS")
+    late = server.submit(prm=B().params(100, 0, 10, 0.7, 20, seed=1), kind=B().BITSP_COORDS, n=30,
+                         coords=I.tsp_coords(31, seed=1), coords2=I.tsp_coords(31, seed=2))
+    for _ in range(12):
+        server.step()
+    assert server.poll(bad)[0] == TIMEOUT
+    for rid in (good, late):
+        status, best, gens, _ = server.poll(rid)
+        assert status == 0 and gens == 20 and np.isfinite(best[0])
+    server.close()
