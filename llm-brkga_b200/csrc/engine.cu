@@ -142,7 +142,9 @@ struct brkga_engine {
     Task* d_tasks_ls = nullptr;
     EvolvePlan evo;            // whole generations in one launch (groups 0: graphs of row and rank launches)
     unsigned long long* evo_words = nullptr;
-    uint32_t evo_step = 0;
+    // the number of the last step that a launch may have taken; a few hundred before the numbers
+    // wrap, so that every longer run passes there
+    uint32_t evo_step = 0xFFFFFF00u;
     int32_t* flag = nullptr;   // set when a wait of one of its launches ran out
 };
 
@@ -561,7 +563,7 @@ int32_t brkga_evolve(brkga_engine* e, int32_t generations) {
         NvtxRange run("generations", e->gen + 1u, e->gen + (unsigned)step);
         err = launch_evolve(e->evo, e->pop.pd->kind, e->pop.sh.n, points_of(*e->pop.pd), e->dd, step, e->evo_step,
                             e->ls_count, e->pop.prm.local_search_moves, e->evo_words, e->pop.sh.Pi, e->stream);
-        if (err == cudaSuccess) e->evo_step += kEvolveSteps * (uint32_t)step;
+        if (err == cudaSuccess) e->evo_step += kEvolveSteps * (uint32_t)step + 1u;  // 1: a number skipped
         if (err == cudaErrorCooperativeLaunchTooLarge) {
             // fewer SMs than the device reports (a partitioned GPU): the launches below do
             e->evo.groups = 0;

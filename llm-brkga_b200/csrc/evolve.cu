@@ -39,6 +39,11 @@ struct EvolveArgs {
     int gens, ls_count;
 };
 
+// Steps are numbered from 1 and wrap past 0, which is what words hold before their first step
+// (and stands for "no step" below).  Neighbours differ in their lowest bit across the wrap too: it
+// picks one of the two buffers of fitness words.
+__host__ __device__ __forceinline__ uint32_t next_step(uint32_t step) { return step == 0xFFFFFFFFu ? 2u : step + 1u; }
+
 __device__ __forceinline__ unsigned long long word_of(uint32_t step, uint32_t v) {
     return ((unsigned long long)step << 32) | v;
 }
@@ -130,7 +135,7 @@ __global__ void __launch_bounds__(T * max_groups(T), 1) evolve_kernel(EvolveArgs
 
     uint32_t step = A.step0, ranked = 0;  // ranked: the step whose rank words hold (0: the sorted array)
     for (int left = A.gens; left > 0; --left) {
-        ++step;
+        step = next_step(step);
         unsigned long long* fw = A.fwords + (size_t)(step & 1u) * P;
         for (int q = g.rg; c0 + grid * q < P; q += groups) {
             const int r = row_of_task(sd, c0 + grid * q);
@@ -171,7 +176,7 @@ __global__ void __launch_bounds__(T * max_groups(T), 1) evolve_kernel(EvolveArgs
         if (TSPJ_ROWS && A.ls_count > 0 && ls_due(sd)) {
             // the best rows searched, each by the CTA that built it, then ranked again
             // (core/solver.hpp:459-461)
-            ++step;
+            step = next_step(step);
             fw = A.fwords + (size_t)(step & 1u) * P;
             for (int q = g.rg; c0 + grid * q < P; q += groups) {
                 const int r = row_of_task(sd, c0 + grid * q);

@@ -118,8 +118,8 @@ struct EvolvePlan {
 bool evolve_plan(int kind, int n, int P, int threads, EvolvePlan* out);
 // `gens` generations of the population at desc (its rows ranked): rows, elite partition, and for
 // TSPJ the local search of ls_count rows where due.  words: 3 P 64-bit words of device memory,
-// zero before the first launch; step0: the steps earlier launches took (kEvolveSteps a
-// generation).
+// zero before the first launch; step0: a number that no step of an earlier launch is past (a launch
+// takes up to kEvolveSteps a generation, and one number more where they wrap).
 constexpr uint32_t kEvolveSteps = 2;
 cudaError_t launch_evolve(const EvolvePlan& p, int kind, int n, int max_points, PopDesc* desc, int gens, uint32_t step0,
                           int ls_count, int ls_moves, unsigned long long* words, int P, cudaStream_t s);
