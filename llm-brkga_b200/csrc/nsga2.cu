@@ -18,11 +18,13 @@
 // for the front that is cut, index, copy); the first P of them.
 #include <algorithm>
 #include <cfloat>
-#include <map>
 #include <cmath>
+#include <cstdlib>
 #include <cstring>
+#include <map>
 #include <mutex>
 #include <string>
+#include <type_traits>
 #include <vector>
 
 #include <cooperative_groups.h>
@@ -768,7 +770,9 @@ __device__ __forceinline__ bool select_active(const PopDesc& d, int mode) {
 // later front is selected.  The points left then get that front's rank + 1 as one last
 // front.  Selection, crowding of every selected point and the ranks kept for the next
 // generation are the same as with every front peeled.  Ranks -> domcnt[0, N).
-constexpr int kPeelThreads = 512, kPeelWarpPoints = 16, kPeelPoints = kPeelThreads / 32 * kPeelWarpPoints;
+constexpr int kPeelThreads = 512;
+// points of a CTA whose warps take S steps of four points
+constexpr int peel_points(int S) { return kPeelThreads / 32 * 4 * S; }
 
 // set bits of x[0, n) (n = 4, 8 or 16): full adders until the logic (two cycles a warp) takes
 // about as long as the counts left (eight cycles a warp)
@@ -799,13 +803,18 @@ __device__ __forceinline__ int count_bits(const uint32_t (&x)[n]) {
 
 __device__ __forceinline__ uint32_t shared_addr(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
 
-template <int WL>
+// S = 4: the rows fit the registers.  S = 8 (half of them spill): clusters of half the size, for
+// devices that cannot place 16 CTAs together (launch_peel).
+template <int WL, int S>
 __global__ void __launch_bounds__(kPeelThreads, 1) nsga_peel_rows_kernel(PopDesc* dd, int mode) {
     dep_wait();
     namespace cg = cooperative_groups;
+    using Part = std::conditional_t<S == 4, uint16_t, uint32_t>;  // a warp's points
     constexpr int NW = 8 * WL;  // words of a mask
+    constexpr int QW = S / 2;   // words of a CTA in each quarter of the points
+    constexpr uint32_t kAll = (1u << S) - 1u;
     __shared__ __align__(16) uint32_t F[4][NW];  // the points of the fronts 0..k in F[k & 3]
-    __shared__ __align__(16) uint16_t out[kPeelThreads / 32];  // the CTA's part of the next mask
+    __shared__ __align__(16) Part out[kPeelThreads / 32];  // the CTA's part of the next mask
     __shared__ __align__(8) uint64_t bar[4];  // of each mask: every CTA's part has arrived
     __shared__ int gave_up[16];  // the last mask that each CTA of the cluster sent before it gave up, or -1
     cg::cluster_group cluster = cg::this_cluster();
@@ -816,11 +825,11 @@ __global__ void __launch_bounds__(kPeelThreads, 1) nsga_peel_rows_kernel(PopDesc
     const int Wmax = d.domW;
     const uint32_t polls = 4u * d.wait_polls;  // a poll of shared memory is shorter than one of L2
     const int t = threadIdx.x, lane = t & 31, warp = t >> 5, sub = lane & 7;
-    // A CTA has pairs of words (64 points each) from the four quarters of the points: a pool's
-    // survivors come in the order of their last fronts, so neighbours are at work together.
-    auto word_of = [&](int quarter) { return 2 * (quarter * csize + crank); };
-    const int word = word_of(warp / 4) + ((warp >> 1) & 1);
-    const int p0 = 32 * word + kPeelWarpPoints * (warp & 1);  // the warp's points; step s: p0 + 4 s + lane / 8
+    // A CTA has QW words from each of the four quarters of the points: a pool's survivors come in
+    // the order of their last fronts, so neighbours are at work together.
+    auto word_of = [&](int quarter) { return QW * (quarter * csize + crank); };
+    const int word = word_of(warp / 4) + (warp & 3) * 4 * S / 32, bit0 = (warp & 3) * 4 * S % 32;
+    const int p0 = 32 * word + bit0;  // the warp's points; step s: p0 + 4 s + lane / 8
 
     if (t < 4) {
         asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(shared_addr(&bar[t])) : "memory");
@@ -833,9 +842,9 @@ __global__ void __launch_bounds__(kPeelThreads, 1) nsga_peel_rows_kernel(PopDesc
         F[0][w] = F[2][w] = F[3][w] = 0u;
     }
     asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
-    uint32_t x[4][WL];
+    uint32_t x[S][WL];
 #pragma unroll
-    for (int st = 0; st < 4; ++st) {
+    for (int st = 0; st < S; ++st) {
         const int p = p0 + 4 * st + (lane >> 3);
 #pragma unroll
         for (int c = 0; c < WL / 4; ++c) {
@@ -846,16 +855,16 @@ __global__ void __launch_bounds__(kPeelThreads, 1) nsga_peel_rows_kernel(PopDesc
         }
     }
     // counts of the points' dominators in a mask, for the steps in `act` (0 for the others)
-    auto dominators_in = [&](const uint32_t* f, uint32_t act, int (&cnt)[4]) {
+    auto dominators_in = [&](const uint32_t* f, uint32_t act, int (&cnt)[S]) {
         uint32_t m[WL];
 #pragma unroll
         for (int c = 0; c < WL / 4; ++c) {
             const uint4 v = *reinterpret_cast<const uint4*>(f + 32 * c + 4 * sub);
             m[4 * c] = v.x, m[4 * c + 1] = v.y, m[4 * c + 2] = v.z, m[4 * c + 3] = v.w;
         }
-        uint32_t pk[2] = {0u, 0u};  // two steps a word
+        uint32_t pk[S / 2] = {};  // two steps a word
 #pragma unroll
-        for (int st = 0; st < 4; ++st) {
+        for (int st = 0; st < S; ++st) {
             if (!((act >> st) & 1u)) continue;
             uint32_t y[WL];
 #pragma unroll
@@ -863,37 +872,43 @@ __global__ void __launch_bounds__(kPeelThreads, 1) nsga_peel_rows_kernel(PopDesc
             pk[st >> 1] |= (uint32_t)count_bits<WL>(y) << (16 * (st & 1));
         }
 #pragma unroll
-        for (int o = 1; o < 8; o <<= 1) {
-            pk[0] += __shfl_xor_sync(0xffffffffu, pk[0], o);
-            pk[1] += __shfl_xor_sync(0xffffffffu, pk[1], o);
-        }
-        cnt[0] = (int)(pk[0] & 0xFFFFu), cnt[1] = (int)(pk[0] >> 16);
-        cnt[2] = (int)(pk[1] & 0xFFFFu), cnt[3] = (int)(pk[1] >> 16);
+        for (int o = 1; o < 8; o <<= 1)
+#pragma unroll
+            for (int h = 0; h < S / 2; ++h) pk[h] += __shfl_xor_sync(0xffffffffu, pk[h], o);
+#pragma unroll
+        for (int st = 0; st < S; ++st) cnt[st] = (int)((pk[st >> 1] >> (16 * (st & 1))) & 0xFFFFu);
     };
     uint32_t ranked = 0u, mine = 0u;  // the warp's points in the fronts so far, in the next one: bit 4 s + lane / 8
-    // the CTA's part of mask b to every CTA, one pair of words a thread
+    // the CTA's part of mask b to every CTA, a quarter's words a thread
     auto deliver = [&](int b) {
         if (t < 4 * csize) {
             const int q = t & 3;
             const uint32_t to = shared_addr(&F[b][word_of(q)]), at = shared_addr(&bar[b]);
             if (t == 0)
-                asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(at), "r"(32 * csize) : "memory");
-            const uint2 v = reinterpret_cast<const uint2*>(out)[q];
+                asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(at), "r"(16 * QW * csize) : "memory");
             uint32_t rto, rat;
             asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(rto) : "r"(to), "r"(t >> 2));
             asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(rat) : "r"(at), "r"(t >> 2));
-            asm volatile("st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.v2.b32 [%0], {%1, %2}, [%3];"
-                         ::"r"(rto), "r"(v.x), "r"(v.y), "r"(rat)
-                         : "memory");
+            if constexpr (QW == 2) {
+                const uint2 v = reinterpret_cast<const uint2*>(out)[q];
+                asm volatile("st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.v2.b32 [%0], {%1, %2}, [%3];"
+                             ::"r"(rto), "r"(v.x), "r"(v.y), "r"(rat)
+                             : "memory");
+            } else {
+                const uint4 v = reinterpret_cast<const uint4*>(out)[q];
+                asm volatile("st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.v4.b32 [%0], {%1, %2, %3, %4}, [%5];"
+                             ::"r"(rto), "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w), "r"(rat)
+                             : "memory");
+            }
         }
     };
     // points of the steps `act` at or below zero and not ranked yet join the next front: the
-    // CTA's 256 bits of mask b gathered, then sent to every CTA
-    auto send_front = [&](int b, uint32_t act, const int (&left)[4]) {
+    // CTA's bits of mask b gathered, then sent to every CTA
+    auto send_front = [&](int b, uint32_t act, const int (&left)[S]) {
         uint32_t bits = 0u;
         if (act) {
 #pragma unroll
-            for (int st = 0; st < 4; ++st) {
+            for (int st = 0; st < S; ++st) {
                 const uint32_t v =
                     __ballot_sync(0xffffffffu, ((act >> st) & 1u) && left[st] <= 0 && p0 + 4 * st + (lane >> 3) < N);
                 bits |= ((v & 1u) | ((v >> 7) & 2u) | ((v >> 14) & 4u) | ((v >> 21) & 8u)) << (4 * st);
@@ -901,7 +916,7 @@ __global__ void __launch_bounds__(kPeelThreads, 1) nsga_peel_rows_kernel(PopDesc
         }
         mine = bits & ~ranked;
         ranked |= mine;
-        if (lane == 0) out[warp] = (uint16_t)ranked;
+        if (lane == 0) out[warp] = (Part)ranked;
         __syncthreads();
         deliver(b);
     };
@@ -920,13 +935,13 @@ __global__ void __launch_bounds__(kPeelThreads, 1) nsga_peel_rows_kernel(PopDesc
         return __syncthreads_and((int)done) != 0;
     };
     __syncthreads();
-    int need[4];  // every point: all its dominators, and once those of the first front are known, them once more
-    dominators_in(F[1], 15u, need);
+    int need[S];  // every point: all its dominators, and once those of the first front are known, them once more
+    dominators_in(F[1], kAll, need);
     asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");  // every CTA's masks and barriers are set up
-    send_front(0, 15u, need);
+    send_front(0, kAll, need);
 
     int survivors = 0, rest = 0, start = 0;
-    int reach[4] = {0, 0, 0, 0};  // listed points at which a step's points may come to zero
+    int reach[S] = {};  // listed points at which a step's points may come to zero
     // thread 0 of the cluster's first CTA records the front table (start of each front in
     // rank order, the cut front) for the grid-wide crowding and placement of mode 0
     int32_t* const ft = (crank == 0 && t == 0) ? d.nft : nullptr;
@@ -950,14 +965,16 @@ __global__ void __launch_bounds__(kPeelThreads, 1) nsga_peel_rows_kernel(PopDesc
             // the steps with a point that may come to zero with this front
             uint32_t act = 0u;
 #pragma unroll
-            for (int st = 0; st < 4; ++st)
+            for (int st = 0; st < S; ++st)
                 act |= __any_sync(0xffffffffu, reach[st] <= total && !((ranked >> (4 * st + (lane >> 3))) & 1u)) ? 1u << st : 0u;
-            int left[4] = {1, 1, 1, 1};
+            int left[S];
+#pragma unroll
+            for (int st = 0; st < S; ++st) left[st] = 1;
             if (act) {
-                int cnt[4];
+                int cnt[S];
                 dominators_in(f, act, cnt);
 #pragma unroll
-                for (int st = 0; st < 4; ++st) {
+                for (int st = 0; st < S; ++st) {
                     if (!((act >> st) & 1u)) continue;
                     if (k == 0) need[st] -= cnt[st];
                     left[st] = need[st] - cnt[st];
@@ -976,10 +993,10 @@ __global__ void __launch_bounds__(kPeelThreads, 1) nsga_peel_rows_kernel(PopDesc
             for (int c = 0; c < NW / 32; ++c) {
                 const int w = 32 * c + lane;
                 const uint32_t v = (k == 0) ? f[w] : f[w] & ~before[w];
-                pre += (w < word) ? __popc(v) : (w == word && (warp & 1)) ? __popc(v & 0xFFFFu) : 0;
+                pre += (w < word) ? __popc(v) : (w == word) ? __popc(v & ((1u << bit0) - 1u)) : 0;
             }
             pre = __reduce_add_sync(0xffffffffu, pre);
-            if (lane < 16 && ((members >> lane) & 1u)) {
+            if (lane < 4 * S && ((members >> lane) & 1u)) {
                 d.domcnt[p0 + lane] = k;
                 if (d.nlist) d.nlist[start + pre + __popc(members & ((1u << lane) - 1u))] = p0 + lane;
             }
@@ -1009,7 +1026,7 @@ __global__ void __launch_bounds__(kPeelThreads, 1) nsga_peel_rows_kernel(PopDesc
     }
     __syncwarp();
     asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
-    if (lane < 16 && p0 + lane < N && !((ranked >> lane) & 1u)) d.domcnt[p0 + lane] = rest;
+    if (lane < 4 * S && p0 + lane < N && !((ranked >> lane) & 1u)) d.domcnt[p0 + lane] = rest;
     // no CTA leaves while another may still send to it
     __syncwarp();
     asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
@@ -1026,18 +1043,46 @@ __global__ void __launch_bounds__(kPeelThreads, 1) nsga_peel_rows_kernel(PopDesc
 
 using PeelFn = void (*)(PopDesc*, int);
 
-// one cluster per population: a CTA for every 256 of its (at most maxN) points
+// CTAs of a peel cluster at most: 16, or the 8 that any device places, where 16 (a non-portable size:
+// as many free SMs in one GPC) cannot be: a partition of the GPU, or BRKGA_PEEL_CLUSTER=8
+static int peel_cluster_limit(PeelFn fn) {
+    const char* v = std::getenv("BRKGA_PEEL_CLUSTER");
+    if (v && std::atoi(v) == 8) return 8;
+    static std::mutex mu;
+    static std::map<int, int> known;  // device -> limit
+    int dev = 0;
+    cudaGetDevice(&dev);
+    std::lock_guard<std::mutex> lk(mu);
+    auto it = known.find(dev);
+    if (it != known.end()) return it->second;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(16);
+    cfg.blockDim = dim3(kPeelThreads);
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = 16;
+    at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    int clusters = 0;
+    cudaError_t e = cudaFuncSetAttribute(reinterpret_cast<const void*>(fn), cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+    if (e == cudaSuccess) e = cudaOccupancyMaxActiveClusters(&clusters, fn, &cfg);
+    if (e != cudaSuccess) cudaGetLastError();
+    return known[dev] = (e == cudaSuccess && clusters > 0) ? 16 : 8;
+}
+
+// one cluster per population: a CTA for every 256 of its (at most maxN) points, 512 where the
+// cluster would be too large for the device
 static cudaError_t launch_peel(PopDesc* dd, int npops, int maxN, int mode, cudaStream_t s) {
+    if (maxN > kMaxPool) return cudaErrorInvalidValue;
+    PeelFn fn = maxN <= 1024   ? nsga_peel_rows_kernel<4, 4>
+                : maxN <= 2048 ? nsga_peel_rows_kernel<8, 4>
+                               : nsga_peel_rows_kernel<16, 4>;
     int csize = 1;
-    while (csize * kPeelPoints < maxN) csize *= 2;
-    if (csize > 16) return cudaErrorInvalidValue;
-    const PeelFn fn = maxN <= 1024   ? nsga_peel_rows_kernel<4>
-                      : maxN <= 2048 ? nsga_peel_rows_kernel<8>
-                                     : nsga_peel_rows_kernel<16>;
-    if (csize > 8) {
-        const cudaError_t e =
-            cudaFuncSetAttribute(reinterpret_cast<const void*>(fn), cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
-        if (e != cudaSuccess) return e;
+    while (csize * peel_points(4) < maxN) csize *= 2;
+    if (csize > 8 && peel_cluster_limit(fn) < csize) {
+        fn = nsga_peel_rows_kernel<16, 8>;
+        csize = 8;
     }
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(npops * csize);
