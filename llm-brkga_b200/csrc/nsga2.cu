@@ -803,6 +803,52 @@ __device__ __forceinline__ int count_bits(const uint32_t (&x)[n]) {
 
 __device__ __forceinline__ uint32_t shared_addr(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
 
+// the current phase of the barrier at `at` has the given parity and completes within `polls` polls
+__device__ __forceinline__ bool mask_arrived(uint32_t at, uint32_t parity, uint32_t polls) {
+    uint32_t done = 0u;
+    for (uint32_t n = 0; n < polls && !done; ++n)
+        asm volatile(
+            "{.reg .pred p;\n\t"
+            "mbarrier.test_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\t"
+            "selp.u32 %0, 1, 0, p;}"
+            : "=r"(done)
+            : "r"(at), "r"(parity)
+            : "memory");
+    return done != 0u;
+}
+
+__device__ __forceinline__ uint32_t shared_addr_in(uint32_t addr, int cta) {
+    uint32_t r;
+    asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(addr), "r"(cta));
+    return r;
+}
+
+// A CTA that gave up at mask k waits here for the words on their way to it; every CTA has sent all
+// that it is going to.  A CTA that sent mask k + 1 waits for it, so it gave up too, and none got
+// further without this CTA's part, which it sends now (its bits do not matter).  CTAs that did
+// not give up have all of mask k, the last one sent then.  (Out of line: in the kernel it took
+// registers that the rows need, 31.0 -> 32.5 us for 4096 points of 12 fronts.)
+template <int QW>
+__device__ __noinline__ void peel_drain(uint32_t masks, int mask_words, uint32_t bars, const int* gave_up, int k, int csize,
+                                        int crank) {
+    const int t = threadIdx.x;
+    int last = k;
+    for (int c = 0; c < csize; ++c) last = max(last, gave_up[c]);
+    if (last > k && t < 4 * csize) {
+        const int q = t & 3, b = last & 3;
+        if (t == 0)
+            asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bars + 8 * b), "r"(16 * QW * csize)
+                         : "memory");
+        const uint32_t to = shared_addr_in(masks + 4 * (b * mask_words + QW * (q * csize + crank)), t >> 2);
+        const uint32_t at = shared_addr_in(bars + 8 * b, t >> 2);
+        for (int w = 0; w < QW; ++w)
+            asm volatile("st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.b32 [%0], %1, [%2];" ::"r"(to + 4 * w),
+                         "r"(0u), "r"(at)
+                         : "memory");
+    }
+    for (int b = k; b <= last; ++b) mask_arrived(bars + 8 * (b & 3), (uint32_t)(b >> 2) & 1u, 4u * kWaitPolls);
+}
+
 // S = 4: the rows fit the registers.  S = 8 (half of them spill): clusters of half the size, for
 // devices that cannot place 16 CTAs together (launch_peel).
 template <int WL, int S>
@@ -816,14 +862,17 @@ __global__ void __launch_bounds__(kPeelThreads, 1) nsga_peel_rows_kernel(PopDesc
     __shared__ __align__(16) uint32_t F[4][NW];  // the points of the fronts 0..k in F[k & 3]
     __shared__ __align__(16) Part out[kPeelThreads / 32];  // the CTA's part of the next mask
     __shared__ __align__(8) uint64_t bar[4];  // of each mask: every CTA's part has arrived
+    __shared__ uint32_t s_polls;  // of one wait (no register to spare for it)
     __shared__ int gave_up[16];  // the last mask that each CTA of the cluster sent before it gave up, or -1
     cg::cluster_group cluster = cg::this_cluster();
     const int csize = (int)cluster.num_blocks(), crank = (int)cluster.block_rank();
     PopDesc& d = dd[blockIdx.x / csize];
+    // (loaded together: one trip to L2, not one for the decision and one for the rest)
+    const volatile PopDesc& vd = d;
+    const int P = vd.P, Wmax = vd.domW;
+    const uint32_t polls = vd.wait_polls;
     if (!select_active(d, mode)) return;  // the same decision in every CTA of the cluster
-    const int N = (mode == 0) ? 2 * d.P : d.P;
-    const int Wmax = d.domW;
-    const uint32_t polls = 4u * d.wait_polls;  // a poll of shared memory is shorter than one of L2
+    const int N = (mode == 0) ? 2 * P : P;
     const int t = threadIdx.x, lane = t & 31, warp = t >> 5, sub = lane & 7;
     // A CTA has QW words from each of the four quarters of the points: a pool's survivors come in
     // the order of their last fronts, so neighbours are at work together.
@@ -836,6 +885,7 @@ __global__ void __launch_bounds__(kPeelThreads, 1) nsga_peel_rows_kernel(PopDesc
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if (t < 16) gave_up[t] = -1;
+    if (t == 0) s_polls = 4u * polls;  // a poll of shared memory is shorter than one of L2
     // (Words past N stay zero in the masks: rows may hold anything there.)
     for (int w = t; w < NW; w += kPeelThreads) {
         F[1][w] = (w < N / 32) ? 0xFFFFFFFFu : (w == N / 32 && (N & 31)) ? (1u << (N & 31)) - 1u : 0u;
@@ -886,9 +936,7 @@ __global__ void __launch_bounds__(kPeelThreads, 1) nsga_peel_rows_kernel(PopDesc
             const uint32_t to = shared_addr(&F[b][word_of(q)]), at = shared_addr(&bar[b]);
             if (t == 0)
                 asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(at), "r"(16 * QW * csize) : "memory");
-            uint32_t rto, rat;
-            asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(rto) : "r"(to), "r"(t >> 2));
-            asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(rat) : "r"(at), "r"(t >> 2));
+            const uint32_t rto = shared_addr_in(to, t >> 2), rat = shared_addr_in(at, t >> 2);
             if constexpr (QW == 2) {
                 const uint2 v = reinterpret_cast<const uint2*>(out)[q];
                 asm volatile("st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.v2.b32 [%0], {%1, %2}, [%3];"
@@ -921,18 +969,9 @@ __global__ void __launch_bounds__(kPeelThreads, 1) nsga_peel_rows_kernel(PopDesc
         deliver(b);
     };
     // mask k is complete; false (in every thread of the CTA) when the wait ran out
-    auto await_front = [&](int k, uint32_t polls) {
-        const uint32_t at = shared_addr(&bar[k & 3]), parity = (uint32_t)(k >> 2) & 1u;
-        uint32_t done = 0u;
-        for (uint32_t n = 0; n < polls && !done; ++n)
-            asm volatile(
-                "{.reg .pred p;\n\t"
-                "mbarrier.test_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\t"
-                "selp.u32 %0, 1, 0, p;}"
-                : "=r"(done)
-                : "r"(at), "r"(parity)
-                : "memory");
-        return __syncthreads_and((int)done) != 0;
+    auto await_front = [&](int k) {
+        const uint32_t left = *static_cast<volatile uint32_t*>(&s_polls);
+        return __syncthreads_and(mask_arrived(shared_addr(&bar[k & 3]), (uint32_t)(k >> 2) & 1u, left)) != 0;
     };
     __syncthreads();
     int need[S];  // every point: all its dominators, and once those of the first front are known, them once more
@@ -949,7 +988,7 @@ __global__ void __launch_bounds__(kPeelThreads, 1) nsga_peel_rows_kernel(PopDesc
     bool stuck = false;
     for (;; ++k) {
         const uint32_t* const f = F[k & 3];
-        if (!await_front(k, polls)) {
+        if (!await_front(k)) {
             stuck = true;
             break;
         }
@@ -1030,15 +1069,7 @@ __global__ void __launch_bounds__(kPeelThreads, 1) nsga_peel_rows_kernel(PopDesc
     // no CTA leaves while another may still send to it
     __syncwarp();
     asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
-    if (stuck) {
-        // Every CTA has sent all that it is going to.  A CTA that sent mask k + 1 waits for it, so
-        // it gave up too, and none got further without this CTA's part.  (CTAs that did not give
-        // up have all of mask k, the last one sent then.)
-        int last = k;
-        for (int c = 0; c < csize; ++c) last = max(last, gave_up[c]);
-        if (last > k) deliver(last & 3);
-        for (int b = k; b <= last; ++b) await_front(b, 4u * kWaitPolls);
-    }
+    if (stuck) peel_drain<QW>(shared_addr(F), NW, shared_addr(bar), gave_up, k, csize, crank);
 }
 
 using PeelFn = void (*)(PopDesc*, int);
