@@ -99,8 +99,6 @@ using namespace bk;
 
 // the longest captured run of plain generations is 2^kMaxRunLog
 constexpr int kMaxRunLog = 4;
-// generations of one evolve launch at most
-constexpr int kEvolveRun = 128;
 
 struct brkga_engine {
     std::mutex mu;
@@ -368,22 +366,6 @@ int32_t brkga_create(brkga_problem* pbh, const brkga_params* params, brkga_engin
         d.gen = 0;
         d.stuck_host = e->flag;
     }
-    // one population: whole generations per launch, where that is the faster way.  The parents of
-    // a generation are then drawn by the CTAs that use them
-    {
-        RowTile forced{};
-        const int threads = forced_tile(sh.n, &forced) ? forced.block : 0;
-        if (!sh.mo && sh.k == 1 && !row_needs_global(sh.n, points_of(*pd), pd->kind) &&
-            evolve_plan(pd->kind, sh.n, sh.Pi, threads, &e->evo)) {
-            if ((st = dalloc(e->pop, &p, (size_t)24 * sh.Pi)) != BRKGA_OK) {
-                destroy_engine(e);
-                return st;
-            }
-            e->evo_words = (unsigned long long*)p;
-            cudaMemsetAsync(p, 0, (size_t)24 * sh.Pi, e->stream);
-            e->hd[0].parents = nullptr;
-        }
-    }
     // TSPJ random 2-opt local search (the reference runs it in its island loop on
     // problems whose config has one: TSPJConfig, configs/tspj_config.hpp:69-136)
     if (!sh.mo && pd->kind == BRKGA_TSPJ && params->local_search_interval > 0 &&
@@ -394,6 +376,22 @@ int32_t brkga_create(brkga_problem* pbh, const brkga_params* params, brkga_engin
         }
         e->ls_count = std::min(params->local_search_individuals, sh.Ei);
         for (auto& d : e->hd) d.ls_interval = params->local_search_interval;
+    }
+    // one population: whole generations per launch, where that is the faster way.  The parents of
+    // a generation are then drawn by the CTAs that use them
+    {
+        RowTile forced{};
+        const int threads = forced_tile(sh.n, &forced) ? forced.block : 0;
+        if (!sh.mo && sh.k == 1 && !row_needs_global(sh.n, points_of(*pd), pd->kind) &&
+            evolve_plan(pd->kind, sh.n, sh.Pi, pd->machines, e->ls_count, params->local_search_moves, threads, &e->evo)) {
+            if ((st = dalloc(e->pop, &p, (size_t)24 * sh.Pi)) != BRKGA_OK) {
+                destroy_engine(e);
+                return st;
+            }
+            e->evo_words = (unsigned long long*)p;
+            cudaMemsetAsync(p, 0, (size_t)24 * sh.Pi, e->stream);
+            e->hd[0].parents = nullptr;
+        }
     }
     // pool allocations and clears are ordered on the engine stream: complete them before
     // the synchronous uploads below touch the memory
@@ -559,7 +557,7 @@ int32_t brkga_evolve(brkga_engine* e, int32_t generations) {
     NvtxRange all("brkga_evolve", e->gen + 1u, e->gen + (unsigned)generations);
     while (e->evo.groups > 0 && left > 0 && err == cudaSuccess) {
         // bounded launches: other streams' work gets its turn between them
-        const int step = std::min(left, kEvolveRun);
+        const int step = std::min(left, e->evo.gens);
         NvtxRange run("generations", e->gen + 1u, e->gen + (unsigned)step);
         err = launch_evolve(e->evo, e->pop.pd->kind, e->pop.sh.n, points_of(*e->pop.pd), e->dd, step, e->evo_step,
                             e->ls_count, e->pop.prm.local_search_moves, e->evo_words, e->pop.sh.Pi, e->stream);

@@ -24,6 +24,7 @@
 // (fitness, row).
 #include <algorithm>
 #include <climits>
+#include <cmath>
 
 #include "kernels.h"
 #include "row_body.cuh"
@@ -230,7 +231,28 @@ static size_t evolve_smem(const EvolvePlan& p, int kind, int n, int P) {
            (p.stage ? points_bytes(n, kind) : 0) + row_align(4u * (uint32_t)round_up(P, 4)) + row_align(12u * rows);
 }
 
-bool evolve_plan(int kind, int n, int P, int threads, EvolvePlan* out) {
+// An SM's cycles for a generation, roughly (3 a key, 1/12 a compare of the ranking, two exchanges;
+// measured, P = 16 384: n = 20 140 K cycles, here 160 K; n = 3000 690 K, here 1.2 M).
+static double generation_cycles(const EvolvePlan& p, int kind, int n, int P, int machines, int ls_count, int ls_moves) {
+    const int T = p.tile.block, rows = (P + p.ctas - 1) / p.ctas;
+    double row = 3.0 * n;
+    if (kind == JOBSCHED)  // a thread passes all jobs for every T-th machine
+        row = std::max(row, 2.0 * n * std::ceil((double)machines / T) * T / 32);
+    double cycles = 10000.0 + rows * (row + P / 12.0);
+    if (ls_count > 0)  // the searched rows may all lie in one CTA; its groups take one at a time
+        cycles += std::ceil((double)std::min(ls_count, rows) / p.groups) * ls_moves * (300.0 + 5.0 * n / T);
+    return cycles;
+}
+
+// A launch holds every SM: other streams wait for its end, and a CTA of it for the others, up to
+// the limit of a wait (about a second).  So launches are bounded by their work: 4.4 ms, which is
+// 128 generations of 2048 rows of 1000 keys (2.3 ms measured), three of 16 384 rows of 8192.  A
+// generation that alone takes longer (a long local search, very many machines) gains nothing
+// from sharing a launch and goes row launch by row launch.
+constexpr double kLaunchCycles = 1 << 23;
+constexpr int kLaunchGens = 128;
+
+bool evolve_plan(int kind, int n, int P, int machines, int ls_count, int ls_moves, int threads, EvolvePlan* out) {
     const int cls = row_class(kind);
     if (kind == EXTERNAL || (cls != ROWS_ORDER && cls != ROWS_TSPJ && cls != ROWS_KEYS)) return false;
     const int sms = device_sm_count(), share = (P + sms - 1) / sms;
@@ -276,6 +298,9 @@ bool evolve_plan(int kind, int n, int P, int threads, EvolvePlan* out) {
     if (best == INT_MAX) return false;
     p.groups = (rows + best - 1) / best;
     p.smem = evolve_smem(p, kind, n, P);
+    const double cycles = generation_cycles(p, kind, n, P, machines, ls_count, ls_moves);
+    if (cycles > kLaunchCycles) return false;
+    p.gens = std::min(kLaunchGens, (int)(kLaunchCycles / cycles));
     *out = p;
     return true;
 }

@@ -112,10 +112,12 @@ struct EvolvePlan {
     int ctas = 0;
     bool stage = false, keep = false;
     size_t smem = 0;
+    int gens = 0;      // generations of a launch at most
 };
 // whether populations of P rows of n keys of this kind run in evolve launches, and how
-// (threads: per row, 0 = chosen by size)
-bool evolve_plan(int kind, int n, int P, int threads, EvolvePlan* out);
+// (threads: per row, 0 = chosen by size; machines: of job scheduling; ls_count rows searched with
+// ls_moves moves each)
+bool evolve_plan(int kind, int n, int P, int machines, int ls_count, int ls_moves, int threads, EvolvePlan* out);
 // `gens` generations of the population at desc (its rows ranked): rows, elite partition, and for
 // TSPJ the local search of ls_count rows where due.  words: 3 P 64-bit words of device memory,
 // zero before the first launch; step0: a number that no step of an earlier launch is past (a launch

@@ -1,0 +1,47 @@
+"""Work that a caller's parameters can make as long as they like does not run inside launches whose
+CTAs wait for each other: with waits of no polls at all (BRKGA_WAIT_POLLS=0) such runs end well,
+where a launch of whole generations gives up."""
+import numpy as np
+import pytest
+
+import instances as I
+import oracle as O
+from test_gpu_engine import oracle_islands
+from test_gpu_ops import B
+from test_gpu_wait_limits import timeout
+
+pytestmark = pytest.mark.gpu
+
+
+def searched(moves):
+    return B().Solver(B().tspj(*I.tspj_instance(20, seed=3)),
+                      B().params(64, 12, 6, 0.7, 6, seed=5, local_search_interval=2, local_search_individuals=3,
+                                 local_search_moves=moves))
+
+
+def test_long_local_search(cuda, monkeypatch):
+    monkeypatch.setenv("BRKGA_WAIT_POLLS", "0")
+    s = searched(5)
+    timeout(s.run)
+    s.close()
+    s = searched(100_000)
+    s.run()
+    assert (np.diff(s.get_fitness_history()) <= 0).all()
+    s.close()
+
+
+def test_many_machines(cuda, monkeypatch):
+    n, P, G = 200, 24, 3
+    jt = (1.0 + np.random.default_rng(4).random(n) * 99.0).astype(np.float32)
+    monkeypatch.setenv("BRKGA_WAIT_POLLS", "0")
+    s = B().Solver(B().jobsched(jt, 40), B().params(P, 4, 2, 0.7, G, seed=6))
+    timeout(s.run)
+    s.close()
+    M = 5_000_000
+    s = B().Solver(B().jobsched(jt, M), B().params(P, 4, 2, 0.7, G, seed=6))
+    s.run()
+    keys, fit = s.get_population()
+    rk, rf, _ = oracle_islands(O.OracleProblem(O.JOBSCHED, n, jt=jt, machines=M), P, 4, 2, 0.7, 6, 1, 0, 0, G, n)
+    np.testing.assert_array_equal(keys, rk)
+    np.testing.assert_array_equal(fit, rf)
+    s.close()
