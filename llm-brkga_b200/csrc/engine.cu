@@ -623,10 +623,13 @@ int32_t brkga_generation(const brkga_engine* e) { return e ? (int32_t)e->gen : B
 
 int32_t brkga_engine_info(brkga_engine* e, int32_t* info, int32_t cap) {
     if (!e || !info || cap < 4) return fail(BRKGA_ERR_INVALID, "need an engine and cap >= 4");
-    info[0] = e->tile.block;
-    info[1] = e->tile.groups;
-    info[2] = e->grid;
-    info[3] = e->stage ? 1 : 0;
+    const bool evo = e->evo.groups > 0;  // e->tile: only for the first population then
+    const RowTile& t = evo ? e->evo.tile : e->tile;
+    info[0] = t.block;
+    info[1] = t.groups;
+    info[2] = evo ? e->evo.ctas : e->grid;
+    info[3] = (evo ? e->evo.stage : e->stage) ? 1 : 0;
+    if (cap > 4) info[4] = evo ? e->evo.gens : 0;
     return BRKGA_OK;
 }
 

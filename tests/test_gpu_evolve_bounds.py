@@ -45,3 +45,27 @@ def test_many_machines(cuda, monkeypatch):
     np.testing.assert_array_equal(keys, rk)
     np.testing.assert_array_equal(fit, rf)
     s.close()
+
+
+def launches(s):
+    out = np.full(5, -1, np.int32)
+    B().check(B().lib().brkga_engine_info(s.h, out.ctypes.data, 5))
+    return tuple(out)
+
+
+@pytest.mark.parametrize("n,P,gens", [(52, 256, 128), (1000, 2048, 128), (8192, 2048, None), (4000, 16384, None)])
+def test_info_of_whole_generations(cuda, n, P, gens):
+    """the launches that evolve, not the first population's; long rows take short ones"""
+    s = B().Solver(B().tsp(I.tsp_coords(n, seed=n)), B().params(P, P // 5, P // 10, 0.7, 2, seed=1))
+    threads, groups, ctas, staged, length = launches(s)
+    assert s.info == (threads, groups, ctas, staged)
+    assert 4 * threads * groups >= n and ctas <= 148 and staged == 1
+    # 4.4 ms at 1.9 GHz and three cycles a key and SM
+    assert length == gens if gens else 1 <= length <= 4.4e-3 * 1.9e9 / (3.0 * n * P / 148)
+    s.close()
+
+
+def test_info_of_separate_launches(cuda):
+    s = B().Solver(B().tsp(I.tsp_coords(100, seed=1)), B().params(200, 40, 20, 0.7, 2, seed=1, num_islands=2))
+    assert launches(s)[4] == 0
+    s.close()
