@@ -1028,6 +1028,9 @@ def main():
                 "scaling": "weak", "vs_baseline": None, "dtype": "f32", "data": "synthetic (seeded uniform coordinates)",
                 "config": workload_config(), "impl": "reference", "cpu_baseline": cb,
                 "e2e": {"value": cb["value"], "unit": "gens/s", "h2d_bytes_per_step": 0, "d2h_bytes_per_step": 0}}
+        if cb["kind"] != "reference":
+            line["unavailable"] = ("the reference's harness (oracle/_ref/libref.so) is not built here; the value is the rate "
+                                   "of this repository's C port of its CPU path, not the reference's own")
         print(json.dumps(line))
         return
 
