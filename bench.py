@@ -10,7 +10,7 @@ tour length kernel + elite-partition sort) of the device-resident solver.
 N > 1 runs N independent replicas (one instance per GPU, no collective: islands and
 instances are independent units), launched one process per GPU by torch.distributed.run.
 One timed step is a stretch of GENS_PER_STEP generations of the device-resident solver
-(one evolve call: cooperative launches of up to 128 generations), with L2 flushed (a 256 MiB
+(one evolve call: cooperative launches of several generations), with L2 flushed (a 256 MiB
 write) before every step, outside its CUDA-event bracket; inside a step the 16 MB
 population stays L2-resident as it does in a solver run.  The JSON line's `value` is
 whole-job generations per second with the population resident in HBM;
@@ -211,6 +211,9 @@ def run_ours(args, rank, world):
     prm = B.params(POP, ELITE, MUTANTS, RHO, E2E_GENERATIONS, seed=reps.seed(SEED_GA), device=dev)
     s = B.Solver(pb, prm)
     s_info = s.info
+    info5 = np.zeros(5, np.int32)  # [4]: generations of one launch at most
+    B.check(B.lib().brkga_engine_info(s.h, info5.ctypes.data, 5))
+    gens_per_launch = int(info5[4])
     s.initialize()
     stream = torch.cuda.ExternalStream(s.stream, device=dev)
     flush = torch.empty(256 * 1024 * 1024 // 4, dtype=torch.float32, device=dev)
@@ -358,8 +361,8 @@ def run_ours(args, rank, world):
                          # kernel's elapsed time)
                          "smem": {"wavefront_pct_of_peak": profile_figure("smem_wavefront_pct_of_peak"),
                                   "source": "profiles/row_kernel_tsp_n1000_p2048.md"}},
-            # one population evolves up to 128 generations a launch
-            "gpu_launches": args.steps * -(-gps // 128),
+            # one population: several generations a launch
+            "gpu_launches": args.steps * (-(-gps // gens_per_launch) if gens_per_launch else 2 * gps),
             # rows decoded and evaluated per generation: children and mutants (elites keep
             # their fitness, as the reference's host path does)
             "individual_evaluations_per_s": value * (POP - ELITE),

@@ -244,12 +244,16 @@ static double generation_cycles(const EvolvePlan& p, int kind, int n, int P, int
     return cycles;
 }
 
-// A launch holds every SM: other streams wait for its end, and a CTA of it for the others, up to
-// the limit of a wait (about a second).  So launches are bounded by their work: 4.4 ms, which is
-// 128 generations of 2048 rows of 1000 keys (2.3 ms measured), three of 16 384 rows of 8192.  A
-// generation that alone takes longer (a long local search, very many machines) gains nothing
-// from sharing a launch and goes row launch by row launch.
-constexpr double kLaunchCycles = 1 << 23;
+// Launches are bounded by their work: a launch that fills the SMs keeps the kernels of other streams
+// waiting to its end.  A launch costs 4.5 us (n = 1000, P = 2048: 8 generations a launch 18.6 us
+// each, 16 18.3, 128 18.0); with 128 of them (2.3 ms) a matrix product beside that solver took
+// 868 us instead of 33 alone, six served requests 194 ms instead of 8, with 9 (0.16 ms) 165 us and
+// 54 ms.  2^20 of the cycles above are 19 generations of 2048 rows of 1000 keys (0.34 ms), three of
+// 2048 rows of 8000.  Populations on less than half the SMs leave the rest to others: 128.  A
+// generation that alone takes 4.4 ms and more (a long local search, very many machines) could
+// outlast the waits of a launch's CTAs, about a second, and gains nothing from sharing one: it
+// goes row launch by row launch.
+constexpr double kLaunchCycles = 1 << 20, kGenerationCycles = 1 << 23;
 constexpr int kLaunchGens = 128;
 
 bool evolve_plan(int kind, int n, int P, int machines, int ls_count, int ls_moves, int threads, EvolvePlan* out) {
@@ -299,8 +303,9 @@ bool evolve_plan(int kind, int n, int P, int machines, int ls_count, int ls_move
     p.groups = (rows + best - 1) / best;
     p.smem = evolve_smem(p, kind, n, P);
     const double cycles = generation_cycles(p, kind, n, P, machines, ls_count, ls_moves);
-    if (cycles > kLaunchCycles) return false;
-    p.gens = std::min(kLaunchGens, (int)(kLaunchCycles / cycles));
+    if (cycles > kGenerationCycles) return false;
+    const double room = 2 * p.ctas < sms ? kGenerationCycles : kLaunchCycles;
+    p.gens = std::max(1, std::min(kLaunchGens, (int)(room / cycles)));
     *out = p;
     return true;
 }
