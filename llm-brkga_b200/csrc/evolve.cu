@@ -261,15 +261,18 @@ bool evolve_plan(int kind, int n, int P, int machines, int ls_count, int ls_move
     if (kind == EXTERNAL || (cls != ROWS_ORDER && cls != ROWS_TSPJ && cls != ROWS_KEYS)) return false;
     const int sms = device_sm_count(), share = (P + sms - 1) / sms;
     // Threads a row, from runs of 300 generations (us a generation; launches = row + rank kernels):
-    // as many as let an SM hold its share of the rows at once, up to one per four keys
-    // (n = 200, P = 1000: 64 threads 7.0, 128 7.7, launches 10.2), at least one per 16 keys
-    // (n = 1500, P = 2048: 128 threads 26.5, 64 28.8, launches 30.0); one warp where a sum in
-    // index order takes most of the time (Rosenbrock n = 1000, P = 2048: 14.9, 64 threads 15.8,
-    // launches 19.3).
+    // as many as let three quarters of an SM hold its share of the rows at once, up to one per
+    // four keys (n = 200, P = 1000: 64 threads 7.0, 128 7.7, launches 10.2), at least one per 16
+    // keys (n = 1500, P = 2048: 128 threads 26.5, 64 28.8, launches 30.0).  Not a whole SM, since a
+    // launch starts only when all its CTAs fit beside what runs: eight engines of n = 2000, P = 256
+    // at once take 52 us a generation of all with 256 threads a row, 80 with the 512 that fill the
+    // SMs, and one alone 10.0 and 9.8 (n = 600, P = 1000: 57 and 91, alone 11.8 and 11.6); half an
+    // SM cost one alone up to a third (n = 300, P = 600: 8.4, 6.3 with this rule).  Kinds without an
+    // order take one warp up to 512 keys, as the sum in index order is most of their time.
     int T = threads;
     if (T == 0) {
         T = 512;
-        while (T > 32 && T * share > kSmThreads) T /= 2;
+        while (T > 32 && T * share > kSmThreads * 3 / 4) T /= 2;
         while (T > 32 && T / 2 * 4 >= n) T /= 2;
         if (cls == ROWS_KEYS) T = 32;
         while (T < 512 && 16 * T < n) T *= 2;

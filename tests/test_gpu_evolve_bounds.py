@@ -8,7 +8,7 @@ import instances as I
 import oracle as O
 from test_gpu_engine import oracle_islands
 from test_gpu_ops import B
-from test_gpu_wait_limits import timeout
+from test_gpu_wait_limits import run_population, timeout
 
 pytestmark = pytest.mark.gpu
 
@@ -73,3 +73,23 @@ def test_info_of_separate_launches(cuda):
     s = B().Solver(B().tsp(I.tsp_coords(100, seed=1)), B().params(200, 40, 20, 0.7, 2, seed=1, num_islands=2))
     assert launches(s)[4] == 0
     s.close()
+
+
+@pytest.mark.parametrize("n,P", [(300, 600), (600, 1000), (700, 500), (1000, 512), (2000, 256), (3000, 256)])
+def test_room_for_other_engines(cuda, n, P):
+    """threads a row: an SM's rows leave room for another launch's CTA, unless the row's length asks
+    for more; and engines at once give what they give one by one"""
+    def solver(seed):
+        return B().Solver(B().tsp(I.tsp_coords(n, seed=n)), B().params(P, P // 5, P // 10, 0.7, 60, seed=seed))
+
+    threads = solver(1).info[0]
+    assert threads * -(-P // 148) <= 768 or 16 * (threads // 2) < n
+    one_by_one = [run_population(solver(i), 40) for i in range(3)]
+    together = [solver(i) for i in range(3)]
+    for s in together:
+        s.initialize()
+        s.evolve(40)
+    for s, want in zip(together, one_by_one):
+        for a, b in zip(s.get_population(), want):
+            np.testing.assert_array_equal(a, b)
+        s.close()
