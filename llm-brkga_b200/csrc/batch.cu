@@ -67,15 +67,16 @@ struct Group {
     // balanced, 8 there cost 8%)
     int task_group = 1;
     int32_t* work = nullptr;  // the row kernel's dynamic dealing counter (launches on `stream`)
-    int32_t* flag = nullptr;  // set when a wait of a member's launches ran out
+    // set when a wait of a member's launches ran out (batches; a server reads its descriptors back
+    // every tick)
+    int32_t* flag = nullptr;
 };
 
 // the group's stream and its zeroed row-dealing counter
 static int32_t group_start(Group& g) {
     cudaError_t e = cudaStreamCreateWithFlags(&g.stream, cudaStreamNonBlocking);
     if (e != cudaSuccess) return cuda_fail(e, "stream");
-    int32_t st = flag_take(&g.flag);
-    if (st == BRKGA_OK) st = dev_alloc((void**)&g.work, 8, g.stream);
+    int32_t st = dev_alloc((void**)&g.work, 8, g.stream);
     if (st != BRKGA_OK) return st;
     if ((e = cudaMemsetAsync(g.work, 0, 8, g.stream)) != cudaSuccess) return cuda_fail(e, "work counter");
     return BRKGA_OK;
@@ -592,6 +593,7 @@ int32_t brkga_batch_create(brkga_problem* const* problems, const brkga_params* p
     b->g.device = dev;
     b->g.task_group = 8;
     int32_t st = group_start(b->g);
+    if (st == BRKGA_OK) st = flag_take(&b->g.flag);
     if (st != BRKGA_OK) {
         brkga_batch_destroy(b);
         return st;
