@@ -179,8 +179,8 @@ int row_max_n() { return 4 * 1024 * 4; }
 int row_max_n_global() { return 1 << 22; }
 
 // The longest rows decoded in shared memory: a counter per key of the tile that covers n and
-// 12 bytes a key.  (The slices above take less; rows in between are long enough for the
-// kernels that spread a row over several CTAs.)
+// 12 bytes a key, which is the line that callers of MO-VRP, batches and the server know.  (The
+// slices above take less: up to 16 384 keys would fit.  Rows in between go to row_kernel_big.)
 bool row_needs_global(int n, int pts, int kind) {
     (void)pts;
     // rows of an external-fitness problem are only built: the global kernel builds them
