@@ -120,7 +120,7 @@ static int32_t upload_tasks(Group& g, const std::vector<Task>& t, Task** out) {
 // build buckets for descriptors [d0, d1) (all of one kind)
 static int32_t build_buckets(Group& g, int d0, int d1, bool nsga, std::vector<Bucket>* out) {
     std::map<std::pair<int, int>, std::vector<int>> by_tile;  // (threads per row, class of kinds)
-    for (int i = d0; i < d1; ++i) by_tile[{pick_tile(g.hd[i].n, g.hd[i].kind).block, row_class(g.hd[i].kind)}].push_back(i);
+    for (int i = d0; i < d1; ++i) by_tile[{pick_tile(g.hd[i].n, g.hd[i].kind, 0).block, row_class(g.hd[i].kind)}].push_back(i);
     for (auto& kv : by_tile) {
         Bucket b;
         b.tile = RowTile{kv.first.first, 1};
@@ -437,7 +437,7 @@ static int32_t make_member(std::shared_ptr<ProblemData> pd, const brkga_params& 
 static cudaError_t init_members(Group& g, const std::vector<Member*>& ms) {
     cudaError_t e = cudaSuccess;
     for (Member* m : ms) {
-        const RowTile t = pick_tile(m->sh.n, m->pd->kind);
+        const RowTile t = pick_tile(m->sh.n, m->pd->kind, 0);
         const int pts = points_of(*m->pd);
         const bool stage = stage_fits(t, m->sh.n, pts, m->pd->kind);
         const int groups = row_groups_per_cta(t, m->sh.n, pts, m->pd->kind, stage, m->sh.Pi);

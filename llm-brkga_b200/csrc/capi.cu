@@ -267,7 +267,7 @@ bool forced_tile(int n, RowTile* t) {
 
 int32_t default_tile(int kind, int n, int pts, int rows, TunedTile* out) {
     RowTile t{};
-    if (!forced_tile(n, &t)) t = pick_tile(n, kind);
+    if (!forced_tile(n, &t)) t = pick_tile(n, kind, rows);
     return tile_setup(t, kind, n, pts, rows, out);
 }
 
@@ -389,7 +389,7 @@ namespace bk {
 // stream-ordered pool and returned to it behind the launch.
 static cudaError_t launch_op_rows(RowLaunch& L, const ProblemData& pd, cudaStream_t st) {
     if (!row_needs_global(pd.n, points_of(pd), pd.kind)) {
-        const RowTile tile = pick_tile(pd.n, pd.kind);
+        const RowTile tile = pick_tile(pd.n, pd.kind, L.ntasks);
         L.stage_xy = stage_fits(tile, pd.n, L.max_points, pd.kind) ? 1 : 0;
         return launch_rows_auto(L, pd.kind, tile, st);
     }

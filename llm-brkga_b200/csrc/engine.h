@@ -159,7 +159,7 @@ int32_t autotune_tile(int kind, int n, int pts, int rows, cudaStream_t stream, F
     cudaEventCreate(&b);
     // each candidate: one warm-up, then the best of three separately timed launches; the
     // default tile (smallest that covers n) is kept unless another is 5% faster
-    const RowTile def = pick_tile(n, kind);
+    const RowTile def = pick_tile(n, kind, rows);
     float best_ms = 1e30f, def_ms = 1e30f;
     TunedTile best, deft;
     for (int c = 0; c < nc; ++c) {

@@ -65,8 +65,8 @@ struct RowLaunch {
     int32_t ls_force;        // MODE_LSEARCH: run whatever the generation (operator); rank q = row q
 };
 
-// the default tile for rows of n keys
-RowTile pick_tile(int n, int kind);
+// the default tile for `rows` rows of n keys (0: a launch's rows fill the GPU whatever the tile)
+RowTile pick_tile(int n, int kind, int rows);
 // every compiled tile whose capacity covers n without being far larger (autotuning set)
 int tile_candidates(int n, RowTile* out, int cap);
 // shared memory bytes for one CTA of the row kernel

@@ -165,13 +165,18 @@ int tile_candidates(int n, RowTile* out, int cap) {
 
 // the default: up to four groups a thread; one warp where a sum in index order takes most of
 // the time, which more threads do not share (job scheduling, n = 1000, P = 2048: 18 us a
-// generation's rows with 32 threads, 21 with 64, 36 with 128)
-RowTile pick_tile(int n, int kind) {
+// generation's rows with 32 threads, 21 with 64, 36 with 128).  Few rows take more threads, up to
+// one for four keys, while an SM's share of the rows takes three quarters of its threads at
+// most: evaluations of n = 921, P = 104 took 11.5 us with 64 threads a row, 6.0 with 256; of TSPJ
+// with 100 cities, P = 2000, 10.3 with 32 and 11.4 with the 64 that would take all.
+RowTile pick_tile(int n, int kind, int rows) {
     if (n > row_max_n()) return RowTile{0, 0};
     if ((kind == JOBSCHED || kind == CONTINUOUS) && tile_covers(32, n)) return RowTile{32, tile_groups(32, n)};
-    for (int b = 32; b < 1024; b *= 2)
-        if (tile_groups(b, n) <= 4) return RowTile{b, tile_groups(b, n)};
-    return RowTile{1024, tile_groups(1024, n)};
+    int b = 32;
+    while (b < 1024 && tile_groups(b, n) > 4) b *= 2;
+    const int sms = device_sm_count(), share = (rows + sms - 1) / sms;
+    while (rows > 0 && b < 1024 && 2 * b * share <= (share == 1 ? kSmThreads : kSmThreads * 3 / 4) && 4 * b < n) b *= 2;
+    return RowTile{b, tile_groups(b, n)};
 }
 
 int row_max_n() { return 4 * 1024 * 4; }
