@@ -88,7 +88,7 @@ __global__ void __launch_bounds__(T * max_groups(T), 1) evolve_kernel(EvolveArgs
     if (threadIdx.x == 0) stuck = 0;
     for (int i = threadIdx.x; i < (int)(sizeof(PopDesc) / 4); i += blockDim.x)
         reinterpret_cast<uint32_t*>(&sd)[i] = reinterpret_cast<const uint32_t*>(A.desc)[i];
-    zero_counters<T>(s, g.tid);
+    if (CLS != ROWS_KEYS) zero_counters<T>(s, g.tid);
     __syncthreads();
     if (sd.stuck) return;  // an earlier launch gave up a wait
     const bool staged = L.stage_xy && has_points(sd.kind);

@@ -258,10 +258,16 @@ __device__ __forceinline__ void row_work(const RowLaunch& L, const PopDesc& sd, 
                     tv += x.y;
                 }
             };
-            take(k.x, 4 * q);
-            take(k.y, 4 * q + 1);
-            take(k.z, 4 * q + 2);
-            take(k.w, 4 * q + 3);
+            if (4 * q + 3 < n) {  // four items by two loads that wait for no key
+                const int4 a = __ldg(reinterpret_cast<const int4*>(sd.wv) + 2 * q);
+                const int4 b = __ldg(reinterpret_cast<const int4*>(sd.wv) + 2 * q + 1);
+                tw += (long long)(k.x > 0.5f ? a.x : 0) + (k.y > 0.5f ? a.z : 0) + (k.z > 0.5f ? b.x : 0) + (k.w > 0.5f ? b.z : 0);
+                tv += (long long)(k.x > 0.5f ? a.y : 0) + (k.y > 0.5f ? a.w : 0) + (k.z > 0.5f ? b.y : 0) + (k.w > 0.5f ? b.w : 0);
+            } else {
+                take(k.x, 4 * q);
+                take(k.y, 4 * q + 1);
+                take(k.z, 4 * q + 2);
+            }
         }
     }
     // rows whose stride has more padding than the last four keys
@@ -367,8 +373,6 @@ __device__ __forceinline__ void row_work(const RowLaunch& L, const PopDesc& sd, 
         } else if (kind == CONTINUOUS) {
             g.sync();
             res[0] = continuous_fitness<T>(n, sd.function, sd.lo, sd.hi, s, g);
-            g.sync();
-            zero_counters<T>(s, t);  // the terms lay over them
         } else {
             g.sync();
             res[0] = jobsched_makespan<T>(n, pts ? pts : sd.jt, sd.machines, s, g);

@@ -56,7 +56,7 @@ __global__ void __launch_bounds__(T * max_groups(T), 1) row_kernel(RowLaunch L) 
     const uint32_t slice = row_slice_bytes(T, L.max_n, L.keep_keys != 0);
     const RowBuf s = row_carve(base + g.rg * slice, T, L.max_n, L.keep_keys != 0);
     float* pts = reinterpret_cast<float*>(base + groups * slice);
-    zero_counters<T>(s, t);
+    if (CLS != ROWS_KEYS) zero_counters<T>(s, t);  // (that class sorts nothing)
     dep_wait();  // shared memory only above this line
 
     // Rows come in runs of one population: its descriptor and coordinates are staged once and
