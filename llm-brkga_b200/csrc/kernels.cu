@@ -2,6 +2,7 @@
 // and island migration.  The fused row kernel is in rows.cu, whole generations in one launch
 // in evolve.cu.  The elite partition ranks (fitness key, row) composites by exact counting
 // across the grid.
+#include <algorithm>
 #include <climits>
 #include <cstdio>
 #include <map>
@@ -566,6 +567,8 @@ __device__ float long_tour(int m, const int32_t* perm, EdgeF edge, float* ed, fl
     return lane_tree(acc, red, t);
 }
 
+// (Rows of an external-fitness problem are only built: as many threads as a row has groups of four
+// keys, and no shared memory.)
 __global__ void __launch_bounds__(kBigBlock, 1) row_kernel_big(RowLaunch L) {
     constexpr int BLOCK = kBigBlock;
     extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -677,7 +680,7 @@ __global__ void __launch_bounds__(kBigBlock, 1) row_kernel_big(RowLaunch L) {
             const int sr = __ldg(sd.sorted + r);
             const float4* a = reinterpret_cast<const float4*>(src + (size_t)sr * ld);
             float4* o = reinterpret_cast<float4*>(dst + (size_t)r * ld);
-            for (int q = t; q < ld / 4; q += BLOCK) o[q] = __ldg(a + q);
+            for (int q = t; q < ld / 4; q += blockDim.x) o[q] = __ldg(a + q);
             if (t < m) dfit[(size_t)r * m + t] = __ldg(sd.fit[cur] + (size_t)sr * m + t);
             __syncthreads();
             continue;
@@ -687,7 +690,7 @@ __global__ void __launch_bounds__(kBigBlock, 1) row_kernel_big(RowLaunch L) {
             const float4* A = reinterpret_cast<const float4*>(src + (size_t)pa * ld);
             const float4* Bv = reinterpret_cast<const float4*>(src + (size_t)pb * ld);
             float4* o = reinterpret_cast<float4*>(dst + (size_t)r * ld);
-            for (int q = t; q < ld / 4; q += BLOCK) {
+            for (int q = t; q < ld / 4; q += blockDim.x) {
                 float k[4] = {0.0f, 0.0f, 0.0f, 0.0f};
                 if (4 * q < n) {
                     float4 a = make_float4(0.f, 0.f, 0.f, 0.f), b = a;
@@ -1066,7 +1069,11 @@ cudaError_t launch_rows_global(const RowLaunch& L, int kind, int grid, cudaStrea
     if (grid > L.ntasks) grid = L.ntasks;
     const cudaError_t e = raise_smem_limit(reinterpret_cast<const void*>(row_kernel_big), big_smem_bytes());
     if (e != cudaSuccess) return e;
-    row_kernel_big<<<grid, kBigBlock, big_smem_bytes(), s>>>(L);
+    // (n = 1000, P = 2048, a generation with the caller's fitness: 56 us with a sort's block and
+    // shared memory)
+    const bool built_only = kind == EXTERNAL;
+    const int block = built_only ? std::min(kBigBlock, round_up((L.max_n + 3) / 4, 32)) : kBigBlock;
+    row_kernel_big<<<grid, block, built_only ? 0 : big_smem_bytes(), s>>>(L);
     return cudaGetLastError();
 }
 
