@@ -436,8 +436,10 @@ __device__ __forceinline__ bool long_argsort(const float* key, int n, uint2* sc,
     // Few chunks: each picks its keys out of the row, read again (L2, coalesced).  Many: the
     // (key, gene) pairs are dealt to their bins in global scratch first, a 32-byte sector for
     // each.  (n = 65 536, 7 chunks: dealing took 90 K cycles a row, 250 K with the scratch not in
-    // L2, and 50 K to read back; the seven passes take 154 K whatever is in L2.)
-    const bool deal = chunks > 12;
+    // L2, and 50 K to read back; the seven passes take 154 K whatever is in L2.  Evaluations of 148
+    // and 512 rows, passes and dealing: n = 130 000 647, 777 and 2547, 2657 us; n = 170 000, 17
+    // chunks, 981, 1029 and 3900, 3569; n = 250 000 1940, 1542 and 7282, 5397.)
+    const bool deal = chunks > 15;
     if (deal) {
         for_keys<T>(key, n, t, [&](float k, int i) {
             sc[atomicAdd(&bins[key_bucket(k, (float)kBigBins, kBigBins)], 1u)] =
