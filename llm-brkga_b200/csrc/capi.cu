@@ -217,7 +217,10 @@ void fill_instance(PopDesc& d, const ProblemData& pd) {
 
 uint32_t wait_polls() {
     const char* v = std::getenv("BRKGA_WAIT_POLLS");
-    return v && *v ? (uint32_t)std::min<unsigned long>(std::strtoul(v, nullptr, 10), kWaitPolls) : kWaitPolls;
+    if (!v || *v < '0' || *v > '9') return kWaitPolls;
+    char* end = nullptr;
+    const unsigned long n = std::strtoul(v, &end, 10);
+    return *end == 0 ? (uint32_t)std::min<unsigned long>(n, kWaitPolls) : kWaitPolls;
 }
 
 int points_of(const ProblemData& pd) {

@@ -162,3 +162,13 @@ def test_server_fails_the_request_alone(cuda, monkeypatch):
         status, best, gens, _ = server.poll(rid)
         assert status == 0 and gens == 20 and np.isfinite(best[0])
     server.close()
+
+
+@pytest.mark.parametrize("value", ["", "many", "-1", "12x", "99999999999999999999"])
+def test_limits_that_are_no_number(cuda, value, monkeypatch):
+    """a value that is no number, or one past the limit, leaves the limit as it is"""
+    monkeypatch.setenv("BRKGA_WAIT_POLLS", value)
+    for make in solvers().values():
+        s = make()
+        s.run()
+        s.close()
